@@ -1543,6 +1543,9 @@ __device__ __forceinline__ bool sweep_tile(const Params& p, const DTile t, const
       for (int q = 0; q < NS; ++q) dst[q] = NET ? out[q] - out[MB_NP + q] : out[q];
     }
   }
+  // the k-face below the first plane reads plane k0-2, whose slot the first staging of the loop overwrites (the TMA
+  // staging has a barrier after its wait)
+  if (t.k0 > 1 && !tma) __syncthreads();
   for (int k = t.k0; k < t.k1; ++k) {
     // the slot of plane k-2 is free: its last readers, the faces of plane k-1, finished before the barrier that
     // preceded pass 2 of plane k-1; so a thread stages plane k+2 as soon as its own pass 2 of plane k-1 is done
