@@ -455,7 +455,8 @@ int mb_autotune(mb_ctx* ctx, const double* P, void* stream);
  * grid (0). Synchronises; invalidates the captured step graph. */
 int mb_set_tuning(mb_ctx* ctx, int kchunk, int persistent);
 
-/* The configuration chosen by mb_autotune (k-chunk 16 and the plain grid before any call) and its sweep time. */
+/* The configuration chosen by mb_autotune and its sweep time. Before any call it reports k-chunk 16 and the plain
+ * grid; the tiles then take the chunk that fills the device for the mesh (16 where the mesh has no 3-D block). */
 int mb_get_tuning(const mb_ctx* ctx, int* kchunk, int* persistent, float* ms);
 
 /* The tile staging of the mixed form's sweep (no counterpart in the reference): tma = 1 (the default) stages each

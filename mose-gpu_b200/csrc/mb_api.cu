@@ -49,12 +49,15 @@ struct mb_ctx {
   std::vector<int> hdims;       // 3 per block of the current mesh (interior extents)
   int kc3 = 16;                 // k-chunk of the sweep tiles of blocks deeper than one cell (mb_set_tuning; the value
                                 // reported by mb_get_tuning: the chunk of the class with the most cells)
-  int kcls[4] = {16, 16, 16, 16};  // the k-chunk per depth class of 3-D blocks (kclass_of), autotuned per class
+  int kcls[4] = {16, 16, 16, 16};  // the k-chunk per depth class of 3-D blocks (kclass_of): chunk_rule's for the mesh
+                                // until mb_autotune or mb_set_tuning fixes them (tuned)
+  bool tuned = false;
   int persistent = 0;           // persistent work-queue sweep of the main tile list (autotuned)
   int persistent_km = 0;        // the same for the tiles of mirrored one-plane blocks (autotuned)
   float tuned_ms = 0.f;         // sweep time of the chosen configuration
   int* d_queue = nullptr;       // tile counter of the persistent sweep
   int ty_sweep = 4;
+  int nsm = 148;                // SMs of the device
   DTile* d_tiles_aux = nullptr;
   int ntiles_aux = 0;
   double* d_scratch = nullptr;  // the engine's own stage buffer (ncell x 5)
@@ -152,6 +155,34 @@ static std::vector<DTile> make_tiles(const std::vector<int>& dims, int ty, int k
         for (int i0 = 1; i0 <= n[0]; i0 += 32) t.push_back(DTile{b, i0, j0, k0, std::min(k0 + kcb, n[2] + 1)});
   }
   return t;
+}
+
+// The k-chunk of the 3-D tiles of a mesh nothing has tuned yet. A sweep runs its tiles in waves of `slots` resident
+// CTAs, and a tile costs its planes plus about two more (the four planes staged and the k-face computed before the
+// first one), so the chunk is the one whose waves x (planes per tile + 2) is smallest; the larger chunk on a tie. A
+// fixed chunk of 16 left a mesh of 53^3 cells on 56 of 444 slots. One B200, a step with chunk 16 and with this rule's:
+// 53^3 mixed 710 and 204 us, 64^3 FP64 2084 and 1357 us, 121x67x45 in two blocks, mixed, 1047 and 472 us; from about
+// 10^6 cells on both fill the chip (192^3 mixed: every chunk from 5 to 64 within 4 %).
+static int chunk_rule(const std::vector<int>& dims, int ty, const std::vector<int>& km, int slots) {
+  long long deepest = 1;
+  for (size_t b = 0; b < dims.size() / 3; ++b)
+    if (km[b] == 0) deepest = std::max<long long>(deepest, dims[3 * b + 2]);
+  int best = 16;
+  double cost = 1e300;
+  for (int kc = (int)std::min<long long>(deepest, 64); kc >= 1; --kc) {
+    long long n = 0, planes = 0;
+    for (size_t b = 0; b < dims.size() / 3; ++b) {
+      const int* d = &dims[3 * b];
+      if (km[b] != 0 || d[2] <= 1) continue;
+      const long long cols = (long long)((d[0] + 31) / 32) * ((d[1] + ty - 1) / ty);
+      n += cols * ((d[2] + kc - 1) / kc);
+      planes += cols * d[2];
+    }
+    if (n == 0) return best;
+    const double c = (double)((n + slots - 1) / slots) * ((double)planes / n + 2.0);
+    if (c < cost) { cost = c; best = kc; }
+  }
+  return best;
 }
 
 // the tile order of a persistent sweep: the largest tiles first, so that the queue ends on small ones
@@ -472,11 +503,21 @@ static int build_tables(mb_ctx* c, const mb_mesh* mesh) {
     for (int a = 0; a < 3; ++a) c->hdims[3 * b + a] = mesh->blk[b].n[a];
   c->hkm.assign(mesh->nblk, 0);
   for (int b = 0; b < mesh->nblk; ++b) c->hkm[b] = mesh->blk[b].group < 0 ? -1 : hb[b].kmirror;
+  if (!c->tuned) {
+    const int kc = chunk_rule(c->hdims, c->ty_sweep, c->hkm, c->p.pgrid);
+    for (int q = 0; q < 4; ++q) c->kcls[q] = kc;
+  }
   std::vector<DTile> ts = make_tiles(c->hdims, c->ty_sweep, c->kc3, 0xe, &c->hkm, 0, c->kcls);
   std::vector<DTile> tk = make_tiles(c->hdims, c->ty_sweep, c->kc3, 0xe, &c->hkm, 1);
   if (c->persistent) sort_by_work(ts, c->hdims, c->ty_sweep);
   if (c->persistent_km) sort_by_work(tk, c->hdims, c->ty_sweep);
-  std::vector<DTile> ta = make_tiles(c->hdims, TY_AUX, 16, 0xe, &c->hkm, -1);
+  // the per-cell kernels (dt, update): 16 planes a tile, fewer where that leaves less than four CTAs per SM
+  int kca = 16;
+  std::vector<DTile> ta = make_tiles(c->hdims, TY_AUX, kca, 0xe, &c->hkm, -1);
+  while (kca > 1 && (int)ta.size() < 4 * c->nsm) {
+    kca /= 2;
+    ta = make_tiles(c->hdims, TY_AUX, kca, 0xe, &c->hkm, -1);
+  }
   // ---- the mixed form reads its geometry in FP32: one conversion per distinct array of this mesh (blocks may
   // share arrays). Every copy is converted afresh (a caller may have replaced an array at the same address);
   // the buffers of the previous mesh are reused where the size matches.
@@ -777,6 +818,7 @@ int mb_init(const mb_mesh* mesh, const mb_scheme* sc, const mb_thermo* th, int d
   {
     int nsm = 0;
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device);
+    c->nsm = std::max(1, nsm);
     const int v = sc->visc ? 1 : 0;
     int occ = MB_BY_FORM(sc->precision, sweep_unit(sc), _occupancy, (v));
     p.pgrid = std::max(1, occ) * std::max(1, nsm);
@@ -1493,6 +1535,7 @@ int mb_autotune(mb_ctx* ctx, const double* P, void* stream) {
     ctx->kcls[c] = kbest;
     if (big < 0 || ccells[c] > ccells[big]) big = c;
   }
+  ctx->tuned = true;
   if (big >= 0) ctx->kc3 = ctx->kcls[big];
   std::vector<DTile> all = make_tiles(ctx->hdims, ty, ctx->kc3, 0xe, &ctx->hkm, 0, ctx->kcls);
   std::vector<DTile> sorted = all;
@@ -1572,6 +1615,7 @@ int mb_set_tuning(mb_ctx* ctx, int kchunk, int persistent) {
   CK(cudaSetDevice(ctx->device));
   CK(cudaDeviceSynchronize());
   ctx->kc3 = kchunk;
+  ctx->tuned = true;
   for (int c = 0; c < 4; ++c) ctx->kcls[c] = kchunk;
   ctx->persistent = persistent;
   std::vector<DTile> use = make_tiles(ctx->hdims, ctx->ty_sweep, kchunk, 0xe, &ctx->hkm, 0);
