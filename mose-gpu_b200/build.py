@@ -29,7 +29,7 @@ UNITS = [("mb_f64.cu", F64), ("mb_irs.cu", F64), ("mb_prec.cu", F64), ("mb_api.c
         [("mb_sweep_f64_rs%d.cu" % r, F64) for r in (0, 1, 4, 12)] + \
         [("mb_sweep_f64f_rs%d.cu" % r, F64F) for r in (0, 1, 4, 12)] + \
         [("mb_sweep_f32_rs%d.cu" % r, F32) for r in (0, 1, 4, 12)]
-DEPS = ["mb_physics.cuh", "mb_engine.cuh", "mb_launch.h", "mb_sweep_inst.inc",
+DEPS = ["mb_pair.cuh", "mb_physics.cuh", "mb_face_fast.cuh", "mb_engine.cuh", "mb_launch.h", "mb_sweep_inst.inc",
         os.path.join("..", "..", "include", "mose_b200.h")]
 
 

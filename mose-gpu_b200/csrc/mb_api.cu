@@ -40,6 +40,8 @@ struct mb_ctx {
   int nrec = 0;
   double* d_tab = nullptr;
   float* d_tabf = nullptr;
+  double* d_tab4 = nullptr;     // the rows interleaved with their differences (Params::tab4)
+  float* d_tab4f = nullptr;     // tab4f, then tabm4f
   DevState* d_st = nullptr;
   DTile* d_tiles_sweep = nullptr;
   int ntiles_sweep = 0;
@@ -78,8 +80,8 @@ struct mb_ctx {
   double* d_ur = nullptr;       // prec: Ur of every row (ghost rows 0), its smoothing buffer, the step's local steps
   double* d_urb = nullptr;
   double* d_dtl = nullptr;
-  struct Geo32 { const double* src; float* buf; long long n; };
-  std::vector<Geo32> geo32;     // FP32 geometry copies of the mixed form (source array, copy, elements)
+  struct Geo32 { const double *src, *src2; float* buf; long long n; };
+  std::vector<Geo32> geo32;     // FP32 geometry copies of the mixed form (source array or pair of arrays, copy, elements)
   int ngroups = 1;              // case clocks
   long long ncell = 0;
   bool dt_valid = false;
@@ -121,7 +123,7 @@ static void free_ctx(mb_ctx* c) {
   if (c->gexec) cudaGraphExecDestroy(c->gexec);
   if (c->graph) cudaGraphDestroy(c->graph);
   void* ptrs[] = {c->d_blk, c->d_recmap, c->d_rec, c->d_grec, c->d_phys, c->d_cubic, c->d_cdst, c->d_csrc,
-                  c->d_pgsrc, c->d_tab, c->d_tabf, c->d_st, c->d_tiles_sweep, c->d_tiles_aux, c->d_scratch, c->d_acc4, c->d_queue, c->d_recflux, c->d_brec, c->d_bcell,
+                  c->d_pgsrc, c->d_tab, c->d_tabf, c->d_tab4, c->d_tab4f, c->d_st, c->d_tiles_sweep, c->d_tiles_aux, c->d_scratch, c->d_acc4, c->d_queue, c->d_recflux, c->d_brec, c->d_bcell,
                   c->d_physf, c->d_cubicf, c->d_tiles_km, c->d_irs, c->d_idst, c->d_isrc, c->d_ur, c->d_urb, c->d_dtl};
   for (void* q : ptrs)
     if (q) cudaFree(q);
@@ -372,6 +374,7 @@ static int build_tables(mb_ctx* c, const mb_mesh* mesh) {
     memset(&d, 0, sizeof(d));
     d.n1 = q.n[0]; d.n2 = q.n[1]; d.n3 = q.n[2];
     d.pi = q.n[0] + 2 * MB_GC; d.pj = q.n[1] + 2 * MB_GC;
+    d.npad = d.pi * d.pj * (q.n[2] + 2 * MB_GC);
     d.grp = q.group;
     d.ndir = (c->ngroups > 1 && q.group >= 0) ? gndir[q.group] : sc->ndir;
     d.boff = q.boff;
@@ -526,14 +529,15 @@ static int build_tables(mb_ctx* c, const mb_mesh* mesh) {
     for (auto& d : hb) {
       const long long pk = d.n3 + 2 * MB_GC;
       const long long npad = (long long)d.pi * d.pj * pk;
-      const long long n[5] = {4LL * (d.n1 + 1) * d.n2 * d.n3, 4LL * d.n1 * (d.n2 + 1) * d.n3, 4LL * d.n1 * d.n2 * (d.n3 + 1),
-                              3 * npad, 9 * npad};
-      const double* src[5] = {d.fm1, d.fm2, d.fm3, d.dl, d.m};
-      float* dst[5];
-      for (int q = 0; q < 5; ++q) {
+      const long long n[4] = {4LL * (d.n1 + 1) * d.n2 * d.n3, 4LL * d.n1 * (d.n2 + 1) * d.n3, 4LL * d.n1 * d.n2 * (d.n3 + 1),
+                              12 * npad};
+      const double* src[4] = {d.fm1, d.fm2, d.fm3, d.m};
+      float* dst[4];
+      for (int q = 0; q < 4; ++q) {
+        const double* src2 = q == 3 ? d.dl : nullptr;  // the cell records hold m and dl: keyed by both
         dst[q] = nullptr;
         for (auto& m : keep)
-          if (m.src == src[q]) dst[q] = m.buf;
+          if (m.src == src[q] && m.src2 == src2 && m.n == n[q]) dst[q] = m.buf;
         if (dst[q]) continue;
         for (auto& m : pool)
           if (m.buf && m.n == n[q]) { dst[q] = m.buf; m.buf = nullptr; break; }
@@ -543,15 +547,16 @@ static int build_tables(mb_ctx* c, const mb_mesh* mesh) {
           c->geo32.clear();
           return MB_E_NOMEM;
         }
-        keep.push_back({src[q], dst[q], n[q]});
-        if (to_float(src[q], dst[q], n[q], c->tstream) != cudaSuccess) {
+        keep.push_back({src[q], src2, dst[q], n[q]});
+        if ((q < 3 ? to_float(src[q], dst[q], n[q], c->tstream)
+                   : cell_records(d.m, d.dl, (float4*)dst[q], npad, c->tstream)) != cudaSuccess) {
           c->geo32 = keep;  // every buffer stays owned by the context
           for (auto& m : pool)
             if (m.buf) c->geo32.push_back(m);
           return MB_E_CUDA;
         }
       }
-      d.fm1f = dst[0]; d.fm2f = dst[1]; d.fm3f = dst[2]; d.dlf = dst[3]; d.mf = dst[4];
+      d.fm1f = dst[0]; d.fm2f = dst[1]; d.fm3f = dst[2]; d.mdf = (const float4*)dst[3];
     }
     for (auto& m : pool)
       if (m.buf) cudaFreeAsync(m.buf, c->tstream);
@@ -741,8 +746,24 @@ int mb_init(const mb_mesh* mesh, const mb_scheme* sc, const mb_thermo* th, int d
     tab[q] = th->cp[q]; tab[nt + q] = th->h[q]; tab[2 * nt + q] = th->mu[q]; tab[3 * nt + q] = th->k[q];
   }
   for (size_t q = 0; q < tab.size(); ++q) tabf[q] = (float)tab[q];
+  // the rows with their differences (Params::tab4, tab4f, tabm4f); the last row starts no interval
+  std::vector<double> tab4(4 * (size_t)nt);
+  std::vector<float> tab4f(8 * (size_t)nt);
+  for (int q = 0; q < nt; ++q) {
+    const int n = std::min(q + 1, nt - 1);
+    const double* t[4] = {th->cp, th->h, th->mu, th->k};
+    for (int v = 0; v < 4; ++v) {
+      const double d = t[v][n] - t[v][q];
+      if (v < 2) { tab4[4 * q + 2 * v] = t[v][q]; tab4[4 * q + 2 * v + 1] = d; }
+      float* f = &tab4f[(v < 2 ? 0 : 4 * (size_t)nt) + 4 * q + 2 * (v & 1)];
+      f[0] = (float)t[v][q];
+      f[1] = (float)d;
+    }
+  }
   TRY(upload(&c->d_tab, tab.data(), tab.size()));
   TRY(upload(&c->d_tabf, tabf.data(), tabf.size()));
+  TRY(upload(&c->d_tab4, tab4.data(), tab4.size()));
+  TRY(upload(&c->d_tab4f, tab4f.data(), tab4f.size()));
   // ---- one clock per case; every case starts with the scheme's stop rule
   if (cudaMalloc((void**)&c->d_st, ngroups * sizeof(DevState)) != cudaSuccess) { free_ctx(c); return MB_E_NOMEM; }
   {
@@ -796,6 +817,9 @@ int mb_init(const mb_mesh* mesh, const mb_scheme* sc, const mb_thermo* th, int d
   memset(&p, 0, sizeof(p));
   p.cp = c->d_tab - th->tmin; p.h = c->d_tab + nt - th->tmin; p.mu = c->d_tab + 2 * nt - th->tmin; p.k = c->d_tab + 3 * nt - th->tmin;
   p.cpf = c->d_tabf - th->tmin; p.hf = c->d_tabf + nt - th->tmin; p.muf = c->d_tabf + 2 * nt - th->tmin; p.kf = c->d_tabf + 3 * nt - th->tmin;
+  p.tab4 = c->d_tab4 - 4 * (long long)th->tmin;
+  p.tab4f = c->d_tab4f - 4 * (long long)th->tmin;
+  p.tabm4f = c->d_tab4f + 4 * (long long)nt - 4 * (long long)th->tmin;
   p.st = c->d_st;
   p.ngroups = ngroups;
   p.nc = c->ncell;
@@ -814,6 +838,10 @@ int mb_init(const mb_mesh* mesh, const mb_scheme* sc, const mb_thermo* th, int d
   p.guard = sc->visc ? 1 : 0; p.state_check = sc->state_check;
   p.cfl = sc->cfl; p.vnn = sc->vnn; p.prandtl = sc->prandtl; p.schmidt = sc->schmidt; p.mco = sc->mco;
   p.n_rk = sc->n_rk; p.irk = 0; p.acc4 = c->d_acc4;
+  p.has_pr = sc->prandtl > 0.0;
+  p.mach_floor = !(sc->mco >= 1.0);
+  p.cd = {p.ri, p.iri, p.mco, p.has_pr ? 1.0 / p.prandtl : 0.0, (double)p.tmin, (double)(p.tmax - 1)};
+  p.cf = {(float)p.cd.ri, (float)p.cd.iri, (float)p.cd.mco, (float)p.cd.ipr, (float)p.cd.t0, (float)p.cd.t1};
   if (cudaMalloc((void**)&c->d_queue, sizeof(int)) != cudaSuccess) { free_ctx(c); return MB_E_NOMEM; }
   {
     int nsm = 0;

@@ -17,6 +17,7 @@
 // and bottom j-faces are computed twice across CTAs. Warps run the face tasks through one call
 // site, which keeps a single copy of the flux code in the kernel.
 #pragma once
+#include "mb_pair.cuh"
 #include "mb_physics.cuh"
 
 namespace mb {
@@ -35,7 +36,8 @@ template <typename R> MB_HD R cvt(double x) { return (R)x; }
 // thermo-cache temperature T = p / (rho Rg) (Mod_Thermo_Cache.f90:327-330). The FP64 forms keep 6 values per cell:
 // rho_s, u, v, w, p, T. The mixed form keeps 5: rho_s, u, v, w, T, and takes p = rho Rg T where it reads it (one
 // value less per cell leaves room in shared memory for the TMA staging buffer at 3 CTAs per SM).
-// Layout [slot][value][jj][ii], ii fastest.
+// Layout: planes of pairs [slot][jj][ii], ii fastest: (u, v), then (w, T), then (rho, p) (6 values) or rho alone (5), so
+// that one shared load brings two values; each kind holds all its slots, so a cell has one offset for all of them.
 constexpr int TXH = 36;
 // The staging of a sweep's state tile, a template parameter of the sweep (STG) chosen per context (mb_autotune,
 // mb_set_staging): STG_PLAIN, per-thread coalesced loads into a 6-value tile (rho_s, u, v, w, p, T) with the k-face
@@ -49,21 +51,6 @@ template <typename R, int STG> struct Stg {
   static constexpr bool kreg = tma;        // k-face fluxes in registers
 };
 
-template <typename R, int TY, int NV_ = 6>
-struct Tile {
-  R* base;
-  R rg;                                              // the gas constant of the single species (5-value tile)
-  static constexpr int NVT = NV_;
-  static constexpr int VS = (TY + 4) * TXH;          // stride between the values of one cell
-  MB_HD int off(int slot, int jj, int ii) const { return slot * NVT * VS + jj * TXH + ii; }
-  // value var (0..4: rho_s, u, v, w, p; 5: T) of the cell at offset o
-  MB_HD R v(int o, int var) const {
-    if (NVT == 6 || var < 4) return base[o + var * VS];
-    if (var == 5) return base[o + 4 * VS];
-    return base[o] * rg * base[o + 4 * VS];
-  }
-};
-
 // the plane slot of plane kk (kk >= -1); the tile of a mirrored one-plane block (KM) holds its one plane only
 template <bool KM = false>
 MB_HD int slot_of(int kk) { return KM ? 0 : (kk + 8) & 3; }
@@ -71,13 +58,53 @@ MB_HD int slot_of(int kk) { return KM ? 0 : (kk + 8) & 3; }
 template <bool KM>
 MB_HD constexpr int tile_planes() { return KM ? 1 : 4; }
 
+template <typename R, int TY, int NV_ = 6, bool KM = false>
+struct Tile {
+  R* base;
+  R rg;                                              // the gas constant of the single species (5-value tile)
+  static constexpr int NVT = NV_;
+  static constexpr int VS = (TY + 4) * TXH;          // cells of a plane
+  static constexpr int NP = tile_planes<KM>() * VS;  // cells of the tile
+  MB_HD int off(int slot, int jj, int ii) const { return slot * VS + jj * TXH + ii; }
+  // value var (0..4: rho_s, u, v, w, p; 5: T) of the cell at offset o
+  MB_HD R v(int o, int var) const {
+    if (var == 1 || var == 2) return base[2 * o + var - 1];
+    if (var == 3) return base[2 * (NP + o)];
+    if (var == 5) return base[2 * (NP + o) + 1];
+    if (NVT == 6) return base[2 * (2 * NP + o) + (var == 4 ? 1 : 0)];
+    const R rho = base[4 * NP + o];
+    return var == 0 ? rho : rho * rg * base[2 * (NP + o) + 1];
+  }
+  __device__ __forceinline__ void put(int o, R rho, R u, R vv, R w, R pr, R T) const {
+    V2<R>* q = reinterpret_cast<V2<R>*>(base);
+    q[o] = mk2<R>(u, vv);
+    q[NP + o] = mk2<R>(w, T);
+    if (NVT == 6) q[2 * NP + o] = mk2<R>(rho, pr);
+    else base[4 * NP + o] = rho;
+  }
+  __device__ __forceinline__ void load_uvwT(int o, V2<R>& A, V2<R>& B) const {
+    const V2<R>* q = reinterpret_cast<const V2<R>*>(base);
+    A = q[o];
+    B = q[NP + o];
+  }
+  __device__ __forceinline__ void load(int o, V2<R>& A, V2<R>& B, V2<R>& C) const {
+    load_uvwT(o, A, B);
+    if (NVT == 6) {
+      C = reinterpret_cast<const V2<R>*>(base)[2 * NP + o];
+    } else {
+      const R rho = base[4 * NP + o];
+      C = mk2<R>(rho, rho * rg * hi2(B));
+    }
+  }
+};
+
 // One interior face of direction d between cell (i,j,k) and its +d neighbour, from the state tile: the
 // convective flux (conv_physics.inc) into out[0..4] and, for Navier-Stokes, the viscous flux
 // (diff_cuf_kernels.inc:11-87 + diff_physics.inc) into out[5..9]. (ii, jj) are the tile coordinates of the
 // cell, sk the slot of plane k. The gradients are built per variable in registers and placed on the
 // axes by d (ia = d; the two tangential axes in increasing order), as the reference's Grad(:, ia/ib/ic).
 template <typename R, int TY, bool VISC, int RS = 0, int LIM = 0, bool KM = false, int NVT = 6>
-MB_HD void face_flux(const Params& p, const DBlk& b, const Tile<R, TY, NVT>& T, int d, int i, int j, int k, int ii,
+MB_HD void face_flux(const Params& p, const DBlk& b, const Tile<R, TY, NVT, KM>& T, int d, int i, int j, int k, int ii,
                      int jj, R* out) {
   // a mirrored block (one cell deep in k, extrapolated k faces) reads its k = 1 plane for the k ghosts
   const int skm = slot_of<KM>(k - 1), sk = slot_of<KM>(k), sk1 = slot_of<KM>(k + 1), sk2 = slot_of<KM>(k + 2);
@@ -93,9 +120,8 @@ MB_HD void face_flux(const Params& p, const DBlk& b, const Tile<R, TY, NVT>& T, 
   for (int s = 0; s < MB_NP; ++s) {
     pm1[s] = T.v(o4[0], s); p0[s] = T.v(o4[1], s); pp1[s] = T.v(o4[2], s); pp2[s] = T.v(o4[3], s);
   }
-  const auto* gdl = Geo<R>::dl(b);
 #pragma unroll
-  for (int q = 0; q < 4; ++q) dlc[q] = (R)ld(gdl + d + 3 * (l0 + (q - 1) * st));
+  for (int q = 0; q < 4; ++q) dlc[q] = Geo<R>::dl(b, l0 + (q - 1) * st, d);
   const auto* f = Geo<R>::fm(b, d) + fmi32(b, d, i, j, k);
   R nx = (R)ld(f), ny = (R)ld(f + 1), nz = (R)ld(f + 2), area = (R)ld(f + 3);
   R bet = (R)1;
@@ -157,12 +183,10 @@ MB_HD void face_flux(const Params& p, const DBlk& b, const Tile<R, TY, NVT>& T, 
     }
   }
   R Mav[3][3];
-  const auto* m1 = Geo<R>::m(b) + 9 * l0;
-  const auto* m2 = Geo<R>::m(b) + 9 * (l0 + st);
 #pragma unroll
   for (int a = 0; a < 3; ++a)
 #pragma unroll
-    for (int q = 0; q < 3; ++q) Mav[a][q] = (R)0.5 * ((R)ld(m1 + a + 3 * q) + (R)ld(m2 + a + 3 * q));
+    for (int q = 0; q < 3; ++q) Mav[a][q] = (R)0.5 * (Geo<R>::m(b, l0, a, q) + Geo<R>::m(b, l0 + st, a, q));
 #pragma unroll
   for (int iv = 0; iv < MB_NP; ++iv) {
     R g1 = G[iv][0], g2 = G[iv][1], g3 = G[iv][2];
@@ -180,6 +204,10 @@ MB_HD void face_flux(const Params& p, const DBlk& b, const Tile<R, TY, NVT>& T, 
   face_thermo<R>(p, frs, fp, drho, dT, tint, tdf0, dcp, dmil, dkl);
   visc_flux<R>(p, G, Pf, nx, ny, nz, area, drho, dT, dcp, dmil, dkl, out + MB_NP);
 }
+
+}  // namespace mb
+#include "mb_face_fast.cuh"
+namespace mb {
 
 // ---------------------------------------------------------------------------------------------
 // The boundary record of the cell (i,j,k) on face F, added into acc (the R_flat row of the cell).
@@ -1191,8 +1219,8 @@ MB_HD R cell_dt_t(const Params& p, const DBlk& b, long long l, const R* pl, R ur
   rotot_rtot(p, pl[0], rho, Rg);
   R Tc = pl[MB_IPR] / (rho * Rg);
   R Sound = f_ss(p, pl[0], pl[MB_IPR], rho, Rg);
-  const auto* m = Geo<R>::m(b) + 9 * l;
-  const auto* dl = Geo<R>::dl(b) + 3 * l;
+  auto m = [&](int a, int q) -> R { return Geo<R>::m(b, l, a, q); };
+  auto dl = [&](int a) -> R { return Geo<R>::dl(b, l, a); };
   R dtc = (R)1e8;
   R Alpha_ = (R)0;
   if (PREC) {
@@ -1202,7 +1230,7 @@ MB_HD R cell_dt_t(const Params& p, const DBlk& b, long long l, const R* pl, R ur
   if (p.dt_additive) {
     R ra_c = (R)0, ra_v = (R)0;
     for (int d = 0; d < b.ndir; ++d) {
-      R m0 = cvt<R>(ld(m + d)), m1 = cvt<R>(ld(m + d + 3)), m2 = cvt<R>(ld(m + d + 6));
+      R m0 = m(d, 0), m1 = m(d, 1), m2 = m(d, 2);
       R gn = rsqrt_(m0 * m0 + m1 * m1 + m2 * m2);
       R vel_ = fabs(pl[MB_IU] * m0 + pl[MB_IV] * m1 + pl[MB_IW] * m2) / gn;
       R lambda = vel_ + Sound;
@@ -1214,7 +1242,7 @@ MB_HD R cell_dt_t(const Params& p, const DBlk& b, long long l, const R* pl, R ur
       if (b.ndir == 3) {
         R g[3][3];
         for (int d = 0; d < 3; ++d)
-          for (int a = 0; a < 3; ++a) g[d][a] = cvt<R>(ld(m + d + 3 * a));
+          for (int a = 0; a < 3; ++a) g[d][a] = m(d, a);
         auto dot = [&](int x, int y) { return g[x][0] * g[y][0] + g[x][1] * g[y][1] + g[x][2] * g[y][2]; };
         auto nr = [&](int x) { return rsqrt_(g[x][0] * g[x][0] + g[x][1] * g[x][1] + g[x][2] * g[x][2]); };
         R c12 = dot(0, 1) / (nr(0) * nr(1)), c13 = dot(0, 2) / (nr(0) * nr(2)), c23 = dot(1, 2) / (nr(1) * nr(2));
@@ -1241,7 +1269,7 @@ MB_HD R cell_dt_t(const Params& p, const DBlk& b, long long l, const R* pl, R ur
     }
   } else {
     for (int d = 0; d < b.ndir; ++d) {
-      R m0 = cvt<R>(ld(m + d)), m1 = cvt<R>(ld(m + d + 3)), m2 = cvt<R>(ld(m + d + 6));
+      R m0 = m(d, 0), m1 = m(d, 1), m2 = m(d, 2);
       R nrm = rsqrt_(m0 * m0 + m1 * m1 + m2 * m2);
       R v0 = m0 / nrm, v1 = m1 / nrm, v2 = m2 / nrm;
       R vel_ = fabs(pl[MB_IU] * v0 + pl[MB_IV] * v1 + pl[MB_IW] * v2);
@@ -1251,7 +1279,7 @@ MB_HD R cell_dt_t(const Params& p, const DBlk& b, long long l, const R* pl, R ur
         vel_ = vel_ * ((R)1 - Alpha_);
         lambda = vel_ + cst_;
       }
-      R dtd = cvt<R>(ld(dl + d)) / lambda * (R)p.cfl;
+      R dtd = dl(d) / lambda * (R)p.cfl;
       dtc = mn(dtd, dtc);
     }
     if (p.visc) {
@@ -1260,7 +1288,7 @@ MB_HD R cell_dt_t(const Params& p, const DBlk& b, long long l, const R* pl, R ur
       wilke(p, pl[0], rho, ti, td, mil, kl);
       R mi = (R)0.0 + mil;
       for (int d = 0; d < b.ndir; ++d) {
-        R dlv = cvt<R>(ld(dl + d));
+        R dlv = dl(d);
         R dtd = (rho * (dlv * dlv) * (R)p.vnn) / mi;
         dtc = mn(dtd, dtc);
       }
@@ -1331,24 +1359,16 @@ __device__ __forceinline__ void report_bad_state(DevState* st, int blk, int i, i
 // Stage plane kk of the tile window: cells (i0-2 .. i0+33) x (j0-2 .. j0+TY+1), those inside the padded block and
 // within jext rows of the interior (jext < 2 for a block one cell deep in j: no j-faces, so only the viscous
 // transverse stencil reads the ghost rows); the others hold zeros.
-template <typename R, int TY, int NVT>
-__device__ __forceinline__ void put_cell(const Params& p, const Tile<R, TY, NVT>& T, int o, R* vals) {
+template <typename R, int TY, int NVT, bool KM>
+__device__ __forceinline__ void put_cell(const Params& p, const Tile<R, TY, NVT, KM>& T, int o, R* vals) {
   R rho, Tc;
   cell_rho_T<R>(p, vals[0], vals[MB_IPR], rho, Tc);
-  constexpr int VS = Tile<R, TY, NVT>::VS;
-#pragma unroll
-  for (int v = 0; v < 4; ++v) T.base[o + v * VS] = vals[v];
-  if (NVT == 6) {
-    T.base[o + 4 * VS] = vals[MB_IPR];
-    T.base[o + 5 * VS] = Tc;
-  } else {
-    T.base[o + 4 * VS] = Tc;
-  }
+  T.put(o, vals[0], vals[MB_IU], vals[MB_IV], vals[MB_IW], vals[MB_IPR], Tc);
 }
 
 template <typename R, int TY, int NVT, bool KM>
 __device__ __forceinline__ void stage_plane(const Params& p, const DBlk& b, const double* __restrict__ P,
-                                            const Tile<R, TY, NVT>& T, int i0, int j0, int kk, int jext) {
+                                            const Tile<R, TY, NVT, KM>& T, int i0, int j0, int kk, int jext) {
   const int sl = slot_of<KM>(kk);
   const long long nc = p.nc;
   for (int c = threadIdx.x; c < TXH * (TY + 4); c += blockDim.x) {
@@ -1360,10 +1380,9 @@ __device__ __forceinline__ void stage_plane(const Params& p, const DBlk& b, cons
       const long long r = row(b, i, j, kk);
 #pragma unroll
       for (int s = 0; s < MB_NP; ++s) vals[s] = cvt<R>(ld(P + r + s * nc));
-      put_cell<R, TY, NVT>(p, T, o, vals);
+      put_cell<R, TY, NVT, KM>(p, T, o, vals);
     } else {
-#pragma unroll
-      for (int v = 0; v < NVT; ++v) T.base[o + v * Tile<R, TY, NVT>::VS] = (R)0;
+      T.put(o, (R)0, (R)0, (R)0, (R)0, (R)0, (R)0);
     }
   }
 }
@@ -1438,7 +1457,7 @@ struct TmaStage {
 // convert the landed raw plane into the tile slot of plane kk (the same cells and values as stage_plane)
 template <typename R, int TY, int NVT, bool KM>
 __device__ __forceinline__ void stage_plane_raw(const Params& p, const DBlk& b, const unsigned char* raw,
-                                                const Tile<R, TY, NVT>& T, int i0, int j0, int kk, int jext) {
+                                                const Tile<R, TY, NVT, KM>& T, int i0, int j0, int kk, int jext) {
   const int sl = slot_of<KM>(kk);
   for (int c = threadIdx.x; c < TXH * (TY + 4); c += blockDim.x) {
     const int jj = c / TXH, ii = c - jj * TXH;
@@ -1450,10 +1469,9 @@ __device__ __forceinline__ void stage_plane_raw(const Params& p, const DBlk& b, 
       const double* src = reinterpret_cast<const double*>(raw + jj * TMA_ROW_BYTES) + sh + ii;
 #pragma unroll
       for (int s = 0; s < MB_NP; ++s) vals[s] = cvt<R>(src[s * TMA_BOX_ROWS]);
-      put_cell<R, TY, NVT>(p, T, o, vals);
+      put_cell<R, TY, NVT, KM>(p, T, o, vals);
     } else {
-#pragma unroll
-      for (int v = 0; v < NVT; ++v) T.base[o + v * Tile<R, TY, NVT>::VS] = (R)0;
+      T.put(o, (R)0, (R)0, (R)0, (R)0, (R)0, (R)0);
     }
   }
 }
@@ -1468,16 +1486,19 @@ __device__ __forceinline__ bool sweep_tile(const Params& p, const DTile t, const
   unsigned char* raw = ts.halo;
   unsigned long long* bar = ts.bar_halo;
   unsigned& phase = ts.ph_halo;
-  constexpr int NF = VISC ? 2 * MB_NP : MB_NP;  // values a face task computes (convective, viscous)
+  // values a face task computes (convective, viscous); the simplified flux path of the solvers with their own unit gives
+  // the net flux (face_fast)
+  constexpr bool PAIR = Fast<R>::on && RS != 0;
+  constexpr int NF = (VISC && !PAIR) ? 2 * MB_NP : MB_NP;
   // values a face keeps in shared memory: both fluxes in the FP64 form (pass 2 sums them in the reference's
   // order); the net flux (convective - viscous) in the mixed form
-  constexpr bool NET = VISC && Fast<R>::on;
+  constexpr bool NET = VISC && Fast<R>::on && !PAIR;
   constexpr int NS = NET ? MB_NP : NF;
   typedef R RowI[33][NS];
   typedef R RowJ[32][NS];
   constexpr int NVT = Stg<R, STG>::nv;
-  Tile<R, TY, NVT> T;
-  T.base = reinterpret_cast<R*>(smem_raw);                                       // [4][NVT][TY+4][36]
+  Tile<R, TY, NVT, KM> T;
+  T.base = reinterpret_cast<R*>(smem_raw);                                       // the state tile
   T.rg = (R)p.ri;
   unsigned char* fbase = smem_raw + sizeof(R) * tile_planes<KM>() * NVT * (TY + 4) * TXH;
   RowI* sFi = reinterpret_cast<RowI*>(fbase);                                     // [TY][33][NS]
@@ -1533,7 +1554,8 @@ __device__ __forceinline__ bool sweep_tile(const Params& p, const DTile t, const
   __syncthreads();
   if (own && t.k0 > 1) {
     R out[NF];
-    face_flux<R, TY, VISC, RS, LIM, KM, NVT>(p, b, T, 2, i, j, t.k0 - 1, tx + 2, ty + 2, out);
+    if constexpr (PAIR) face_fast<R, TY, VISC, RS, LIM, KM, NVT>(p, b, T, 2, i, j, t.k0 - 1, tx + 2, ty + 2, out);
+    else face_flux<R, TY, VISC, RS, LIM, KM, NVT>(p, b, T, 2, i, j, t.k0 - 1, tx + 2, ty + 2, out);
     if (KREG) {
 #pragma unroll
       for (int q = 0; q < NS; ++q) kdn[q] = NET ? out[q] - out[MB_NP + q] : out[q];
@@ -1588,7 +1610,8 @@ __device__ __forceinline__ bool sweep_tile(const Params& p, const DTile t, const
       }
       if (d < 0) continue;
       R out[NF];
-      face_flux<R, TY, VISC, RS, LIM, KM, NVT>(p, b, T, d, fi, fj, k, ii, jj, out);
+      if constexpr (PAIR) face_fast<R, TY, VISC, RS, LIM, KM, NVT>(p, b, T, d, fi, fj, k, ii, jj, out);
+      else face_flux<R, TY, VISC, RS, LIM, KM, NVT>(p, b, T, d, fi, fj, k, ii, jj, out);
       if (KREG && task == 4) {
 #pragma unroll
         for (int q = 0; q < NS; ++q) kup[q] = NET ? out[q] - out[MB_NP + q] : out[q];
@@ -1629,7 +1652,7 @@ __device__ __forceinline__ bool sweep_tile(const Params& p, const DTile t, const
           if (hr) a = a + hr[s];
           if (hl) a = a - hl[s];
         }
-        if (VISC && !NET) {
+        if (VISC && !NET && !PAIR) {
           if (fr) a = a - fr[MB_NP + s];
           if (fl) a = a + fl[MB_NP + s];
           if (gr) a = a - gr[MB_NP + s];

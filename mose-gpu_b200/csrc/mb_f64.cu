@@ -118,6 +118,20 @@ cudaError_t to_float(const double* src, float* dst, long long n, cudaStream_t s)
   return cudaGetLastError();
 }
 
+__global__ void k_cell_records(const double* __restrict__ m, const double* __restrict__ dl, float4* __restrict__ dst,
+                               long long npad) {
+  for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < 3 * npad; q += (long long)gridDim.x * blockDim.x) {
+    const long long a = q / npad, l = q - a * npad;
+    const double* c = m + 9 * l + a;
+    dst[q] = make_float4((float)c[0], (float)c[3], (float)c[6], (float)dl[3 * l + a]);
+  }
+}
+
+cudaError_t cell_records(const double* m, const double* dl, float4* dst, long long npad, cudaStream_t s) {
+  k_cell_records<<<1184, 256, 0, s>>>(m, dl, dst, npad);
+  return cudaGetLastError();
+}
+
 __global__ void k_reset_dt(Params p, int only_group) {
   for (int g = threadIdx.x; g < p.ngroups; g += blockDim.x)
     if (only_group < 0 || g == only_group) p.st[g].dtmin_bits = (unsigned long long)__double_as_longlong(1e300);

@@ -46,21 +46,38 @@ struct DBlk {
   int rmap[6];          // offset of each face's record map in Params::rec_map (-1: none)
   long long boff;
   const double *fm1, *fm2, *fm3, *dl, *m, *vol;
-  // FP32 copies of the face and cell geometry, made once by mb_init for the mixed form (null otherwise)
-  const float *fm1f, *fm2f, *fm3f, *dlf, *mf;
+  // FP32 copies of the face and cell geometry, made once by mb_init for the mixed form (null otherwise): the face
+  // records as they are, the cell metrics as one 16-byte record per cell and computational direction a,
+  // mdf[a * npad + cell] = (m(a, 1..3), dl(a)): a warp reads 32 consecutive records of a direction in four 128-byte
+  // lines with one load, where the layouts (9, cells) and (3, cells) took four scalar loads of nine and three lines
+  const float *fm1f, *fm2f, *fm3f;
+  const float4* mdf;
+  int npad;             // padded cells of the block
 };
+
+template <typename T>
+MB_HD T ldg_(const T* q) {
+#ifdef __CUDA_ARCH__
+  return __ldg(q);
+#else
+  return *q;
+#endif
+}
 
 // the geometry arrays in the flux arithmetic type
 template <typename R> struct Geo;
 template <> struct Geo<double> {
   MB_HD static const double* fm(const DBlk& b, int d) { return d == 0 ? b.fm1 : (d == 1 ? b.fm2 : b.fm3); }
-  MB_HD static const double* dl(const DBlk& b) { return b.dl; }
-  MB_HD static const double* m(const DBlk& b) { return b.m; }
+  // the metric m(a, q) and the cell size dl(a) of padded cell l
+  MB_HD static double m(const DBlk& b, long long l, int a, int q) { return ldg_(b.m + 9 * l + a + 3 * q); }
+  MB_HD static double dl(const DBlk& b, long long l, int a) { return ldg_(b.dl + 3 * l + a); }
 };
 template <> struct Geo<float> {
   MB_HD static const float* fm(const DBlk& b, int d) { return d == 0 ? b.fm1f : (d == 1 ? b.fm2f : b.fm3f); }
-  MB_HD static const float* dl(const DBlk& b) { return b.dlf; }
-  MB_HD static const float* m(const DBlk& b) { return b.mf; }
+  MB_HD static float m(const DBlk& b, long long l, int a, int q) {
+    return ldg_(reinterpret_cast<const float*>(b.mdf + a * (long long)b.npad + l) + q);
+  }
+  MB_HD static float dl(const DBlk& b, long long l, int a) { return ldg_(&b.mdf[a * (long long)b.npad + l].w); }
 };
 
 struct DRec {
@@ -92,6 +109,14 @@ struct DevState {
   double rampf;                   // cfl-rise-threshold factor of the current step (1 without a ramp)
 };
 
+// the constants of the simplified flux path in the flux arithmetic type
+template <typename R>
+struct FluxCst {
+  R ri, iri;   // gas constant and its reciprocal
+  R mco, ipr;  // Mco, 1 / Prandtl (0 without one)
+  R t0, t1;    // first and last table row that starts an interval
+};
+
 struct Params {
   const DBlk* blk;
   const int* rec_map;
@@ -99,6 +124,13 @@ struct Params {
   const long long* pgsrc;  // [connection][6]: the rows of P that bc_pg(:,1:6) of the connection record copies
   const double *cp, *h, *mu, *k;      // FP64 tables, indexed by the table row (pointer shifted by -tmin)
   const float *cpf, *hf, *muf, *kf;   // FP32 copies for the mixed form
+  // the rows interleaved with their differences (the row shifted by -tmin like the others): (cp, dcp, h, dh) in FP64 and
+  // FP32, (mu, dmu, k, dk) in FP32; a lookup is one or two 16-byte loads
+  const double* tab4;
+  const float *tab4f, *tabm4f;
+  FluxCst<double> cd;
+  FluxCst<float> cf;
+  int has_pr, mach_floor;             // Prandtl > 0; Mco < 1
   DevState* st;            // one clock per case: st[DBlk::grp]
   int ngroups;
   long long nc;
@@ -155,6 +187,10 @@ template <> struct Tab<float> {
   MB_HD static const float* k(const Params& p) { return p.kf; }
 };
 
+template <typename R> struct Cst;
+template <> struct Cst<double> { MB_HD static const FluxCst<double>& of(const Params& p) { return p.cd; } };
+template <> struct Cst<float> { MB_HD static const FluxCst<float>& of(const Params& p) { return p.cf; } };
+
 template <typename R> MB_HD R rsqrt_(R x);
 template <> MB_HD double rsqrt_(double x) { return sqrt(x); }
 template <> MB_HD float rsqrt_(float x) { return sqrtf(x); }
@@ -192,20 +228,8 @@ MB_HD int fmi32(const DBlk& b, int d, int i, int j, int k) {
   if (d == 1) return 4 * ((i - 1) + b.n1 * (j + (b.n2 + 1) * (k - 1)));
   return 4 * ((i - 1) + b.n1 * ((j - 1) + b.n2 * k));
 }
-MB_HD double ld(const double* p) {
-#ifdef __CUDA_ARCH__
-  return __ldg(p);
-#else
-  return *p;
-#endif
-}
-MB_HD float ld(const float* p) {
-#ifdef __CUDA_ARCH__
-  return __ldg(p);
-#else
-  return *p;
-#endif
-}
+MB_HD double ld(const double* p) { return ldg_(p); }
+MB_HD float ld(const float* p) { return ldg_(p); }
 
 // min / max with the semantics of std::min / std::max of the CPU restatement ((b < a) ? b : a and
 // (a < b) ? b : a): the same operand is returned for equal values, so signed zeros match as well
