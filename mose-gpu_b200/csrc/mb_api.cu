@@ -196,6 +196,12 @@ static void sort_by_work(std::vector<DTile>& t, const std::vector<int>& dims, in
   std::stable_sort(t.begin(), t.end(), [&](const DTile& a, const DTile& b) { return w(a) > w(b); });
 }
 
+// The launches of a stage are chained (launch_chained) on meshes of at most one tile per SM. On more, the CTAs that a
+// kernel places while the one before still runs go where slots happen to be free, and the uneven placement costs more
+// than the gaps: one B200, a step of 1-D, 1000 cells (32 tiles) 68 us unchained and 60 us chained, but 53^3 mixed (378
+// tiles) 160 and 199 us, 2-D 301^2 (380 tiles) 86 and 88 us.
+static void set_chain(mb_ctx* c) { c->p.chain = c->ntiles_sweep + c->ntiles_km <= c->nsm; }
+
 static const double RKC[3][3] = {{1.0, 0.0, 0.0}, {1.0, 0.50, 0.0}, {1.0, 0.25, 2.0 / 3.0}};  // Lib_RK.f90:6-9
 
 // rk_coeff of stage irk (the SSP forms); RK4 carries its own weights in the update (cons_update)
@@ -469,6 +475,7 @@ static int build_tables(mb_ctx* c, const mb_mesh* mesh) {
   };
   auto guide = [](int F, int ax) { int d = (F + 1) / 2 - 1; return ax == d ? ((F % 2) ? 1 : -1) : 0; };
   std::vector<long long> cdst, csrc, pgsrc;
+  bool deep_donors = true;  // every copied row is an interior cell of its donor
   for (int q = 0; q < mesh->nconn; ++q) {
     const mb_conn& cn = mesh->conn[q];
     if (cn.rec < 0 || cn.rec >= mesh->nrec || cn.bs < 0 || cn.bs >= mesh->nblk || mesh->rec[cn.rec].conn != q)
@@ -480,6 +487,11 @@ static int build_tables(mb_ctx* c, const mb_mesh* mesh) {
                            cn.ks + guide(cn.fs, 2) * (g - 1)));
     }
     const int I = cn.is, J = cn.js, K = cn.ks;
+    for (int g = 0; g < MB_GC; ++g) {
+      const int di = I + guide(cn.fs, 0) * g, dj = J + guide(cn.fs, 1) * g, dk = K + guide(cn.fs, 2) * g;
+      const int32_t* dn = mesh->blk[cn.bs].n;
+      if (di < 1 || di > dn[0] || dj < 1 || dj > dn[1] || dk < 1 || dk > dn[2]) deep_donors = false;
+    }
     int t[4][3];
     if (cn.fs <= 2) {
       int a[4][3] = {{I, J - cn.d11, K - cn.d12}, {I, J + cn.d11, K + cn.d12}, {I, J - cn.d21, K - cn.d22}, {I, J + cn.d21, K + cn.d22}};
@@ -637,6 +649,7 @@ static int build_tables(mb_ctx* c, const mb_mesh* mesh) {
     return MB_E_NOMEM;
   c->ntiles_sweep = (int)ts.size();
   c->ntiles_aux = (int)ta.size();
+  set_chain(c);
   Params& p = c->p;
   p.blk = c->d_blk; p.rec_map = c->d_recmap; p.rec = c->d_rec; p.pgsrc = c->d_pgsrc;
   p.recflux = c->d_recflux;
@@ -644,6 +657,7 @@ static int build_tables(mb_ctx* c, const mb_mesh* mesh) {
   g.rec = c->d_grec; g.phys = c->d_phys; g.nphys = (int)phys.size(); g.cubic = c->d_cubic; g.ncubic = (int)cubic.size();
   g.cdst = c->d_cdst; g.csrc = c->d_csrc; g.ncopy = (int)cdst.size(); g.pgsrc = c->d_pgsrc; g.nconn = mesh->nconn;
   g.ordered = ordered;
+  g.fused = !ordered && deep_donors;
   for (int f = 0; f < 3; ++f) { g.phys_off[f] = po[f]; g.cubic_off[f] = co[f]; }
   c->gf = g;
   c->gf.phys = c->d_physf; c->gf.nphys = (int)physf.size(); c->gf.cubic = c->d_cubicf; c->gf.ncubic = (int)cubicf.size();
@@ -848,9 +862,9 @@ int mb_init(const mb_mesh* mesh, const mb_scheme* sc, const mb_thermo* th, int d
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device);
     c->nsm = std::max(1, nsm);
     const int v = sc->visc ? 1 : 0;
-    int occ = MB_BY_FORM(sc->precision, sweep_unit(sc), _occupancy, (v));
+    int occ = MB_BY_FORM(sc->precision, sweep_unit(sc), _occupancy, (v, sc->limiter));
     p.pgrid = std::max(1, occ) * std::max(1, nsm);
-    int occ_km = MB_BY_FORM(sc->precision, sweep_unit(sc), _occupancy_km, (v));
+    int occ_km = MB_BY_FORM(sc->precision, sweep_unit(sc), _occupancy_km, (v, sc->limiter));
     p.pgrid_km = std::max(1, occ_km) * std::max(1, nsm);
   }
   p.queue = nullptr;
@@ -858,8 +872,8 @@ int mb_init(const mb_mesh* mesh, const mb_scheme* sc, const mb_thermo* th, int d
   TRY(build_tables(c, mesh));
   if (getenv("MB_REPORT")) {
     const int v = sc->visc ? 1 : 0;
-    int occ = MB_BY_FORM(sc->precision, sweep_unit(sc), _occupancy, (v));
-    int occ_km = MB_BY_FORM(sc->precision, sweep_unit(sc), _occupancy_km, (v));
+    int occ = MB_BY_FORM(sc->precision, sweep_unit(sc), _occupancy, (v, sc->limiter));
+    int occ_km = MB_BY_FORM(sc->precision, sweep_unit(sc), _occupancy_km, (v, sc->limiter));
     fprintf(stderr, "[mose_b200] sweep: %s, %d threads per CTA, %d CTAs per SM (%d for one-plane blocks), %d + %d tiles\n",
             sc->precision == MB_PREC_MIXED ? "mixed" : (sc->precision == MB_PREC_FP64_FAST ? "fp64 fast" : "fp64"),
             32 * c->ty_sweep, occ, occ_km, c->ntiles_sweep, c->ntiles_km);
@@ -1616,6 +1630,7 @@ int mb_autotune(mb_ctx* ctx, const double* P, void* stream) {
   if ((rc = upload(&ctx->d_tiles_km, use_km.data(), use_km.size())) != MB_OK) return rc;
   ctx->ntiles_sweep = (int)use.size();
   ctx->ntiles_km = (int)use_km.size();
+  set_chain(ctx);
   CK(cudaStreamSynchronize(0));
   if (ctx->gexec) { cudaGraphExecDestroy(ctx->gexec); ctx->gexec = nullptr; }
   if (ctx->graph) { cudaGraphDestroy(ctx->graph); ctx->graph = nullptr; }
@@ -1653,6 +1668,7 @@ int mb_set_tuning(mb_ctx* ctx, int kchunk, int persistent) {
   int rc = upload(&ctx->d_tiles_sweep, use.data(), use.size());
   if (rc != MB_OK) return rc;
   ctx->ntiles_sweep = (int)use.size();
+  set_chain(ctx);
   if (ctx->gexec) { cudaGraphExecDestroy(ctx->gexec); ctx->gexec = nullptr; }
   if (ctx->graph) { cudaGraphDestroy(ctx->graph); ctx->graph = nullptr; }
   ctx->gP = nullptr;

@@ -26,6 +26,14 @@ struct DTile {
   int blk, i0, j0, k0, k1;  // cells i0..i0+31, j0..j0+TY-1, planes k0..k1-1 (1-based)
 };
 
+// ---- launches of a stage in a chain of programmatic dependences: a kernel starts by letting the next one of the stream
+// launch (pdl_next) and, before it touches anything an earlier kernel wrote, waits until the one before has ended and
+// its writes are visible (pdl_wait; every thread of every kernel of the chain, so that the end of one kernel implies the
+// end of all before it). What it does before the wait reads only the mesh tables, which no kernel writes. Only
+// on the smallest meshes (Params::chain).
+__device__ __forceinline__ void pdl_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 enum { MODE_RESIDUAL = 0, MODE_UPDATE = 1 };
 
 template <typename R> MB_HD R cvt(double x) { return (R)x; }
@@ -973,6 +981,8 @@ MB_HD void bc_record(const Params& p, const DBlk& b, const double* __restrict__ 
 template <typename R, bool VISC, int RS, int LIM, int VAR = 0>
 __global__ void __launch_bounds__(128) k_records(Params p, const int* __restrict__ brec, const int* __restrict__ bcell,
                                                int nrec, const double* __restrict__ P) {
+  pdl_next();
+  pdl_wait();
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= nrec) return;
   const int rid = brec[q];
@@ -1790,6 +1800,7 @@ k_sweep(Params p, const DTile* __restrict__ tiles, const double* __restrict__ Pi
   __shared__ int s_next;
   __shared__ __align__(8) unsigned long long s_bar;  // TMA staging: the mbarrier of the landing plane
   static_assert(TY <= 8, "one residual slot per warp");
+  pdl_next();
   TmaStage ts{nullptr, &s_bar, 0u};
   if (Stg<R, STG>::tma) {  // the staging buffer after the tile and the flux buffers, 128-byte aligned
     unsigned char* q = smem_raw + sweep_smem_core<R, TY, VISC, STG, KM>();
@@ -1803,6 +1814,7 @@ k_sweep(Params p, const DTile* __restrict__ tiles, const double* __restrict__ Pi
       __syncthreads();
     }
   }
+  pdl_wait();
   if (!p.queue) {
     sweep_tile<R, TY, VISC, MODE, RS, LIM, KM, STG>(p, tiles[blockIdx.x], Pin, Pold, Pout, Rout, rkc, last, smem_raw,
                                                      sred, s_res, ts);

@@ -28,6 +28,9 @@ struct GhostLists {
   // holding the records whose opposite-face partner on the same column comes earlier in record order; each pass then
   // runs as two launches (only on blocks with an axis of at most two cells does the order change values)
   int ordered;
+  // fused != 0: no ghost is computed from another ghost of the fill (ordered == 0, and every connection copies interior
+  // cells of its donor: the donor is at least two cells deep along its axis), so that one launch fills all of them
+  int fused;
   int phys_off[3];
   int cubic_off[3];
 };
@@ -37,6 +40,26 @@ constexpr int TY_F32 = 8;    // tile rows of the mixed sweep (256 threads)
 constexpr int MINB_F64 = 2;  // resident CTAs per SM the FP64 sweep's registers must allow
 constexpr int MINB_F32 = 3;  // resident CTAs per SM the mixed sweep's registers must allow (80 registers)
 constexpr int TY_AUX = 8;    // tile rows of the per-cell kernels (dt, update)
+
+#ifdef __CUDACC__
+// a launch of the stage's chain (pdl_next, pdl_wait of mb_engine.cuh); chain = false (Params::chain): an ordinary launch,
+// after the end of the one before
+template <typename... K, typename... A>
+static inline cudaError_t launch_chained(bool chain, void (*kernel)(K...), unsigned grid, unsigned block, size_t smem,
+                                         cudaStream_t s, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = chain ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, K(args)...);
+}
+#endif
 
 #define MB_CAT2(a, b) a##b
 #define MB_CAT(a, b) MB_CAT2(a, b)
@@ -49,8 +72,8 @@ constexpr int TY_AUX = 8;    // tile rows of the per-cell kernels (dt, update)
                              cudaStream_t s);                                                                    \
   cudaError_t name##_dt(const Params& p, const DTile* tiles, int ntiles, const double* P, int only_group,       \
                         cudaStream_t s);                                                                         \
-  int name##_occupancy(int visc);                                                                            \
-  int name##_occupancy_km(int visc);
+  int name##_occupancy(int visc, int lim);                                                                       \
+  int name##_occupancy_km(int visc, int lim);
 MB_DECLARE_SWEEP(sweep_f64_rs1)
 MB_DECLARE_SWEEP(sweep_f64_rs4)
 MB_DECLARE_SWEEP(sweep_f64_rs12)

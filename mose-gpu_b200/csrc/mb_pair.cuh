@@ -19,13 +19,13 @@ template <> __device__ __forceinline__ V2<float> mk2(float x, float y) {
 __device__ __forceinline__ double lo2(const V2<double>& a) { return a.x; }
 __device__ __forceinline__ double hi2(const V2<double>& a) { return a.y; }
 __device__ __forceinline__ float lo2(const V2<float>& a) {
-  float x, y;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a.q));
+  float x;
+  asm("{\n .reg .b32 t;\n mov.b64 {%0, t}, %1;\n}" : "=f"(x) : "l"(a.q));
   return x;
 }
 __device__ __forceinline__ float hi2(const V2<float>& a) {
-  float x, y;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a.q));
+  float y;
+  asm("{\n .reg .b32 t;\n mov.b64 {t, %0}, %1;\n}" : "=f"(y) : "l"(a.q));
   return y;
 }
 template <typename R> __device__ __forceinline__ V2<R> dup2(R x) { return mk2<R>(x, x); }
