@@ -35,8 +35,7 @@ struct mb_ctx {
   long long* d_csrc = nullptr;
   long long* d_pgsrc = nullptr;
   double* d_recflux = nullptr;  // boundary-record contributions [nrec][10] (flux type)
-  int* d_brec = nullptr;        // records in type order (the record kernel's work list)
-  int* d_bcell = nullptr;       // their blk, i, j, k, face
+  RecWork* d_work = nullptr;    // records in type order (the record kernel's work list)
   int nrec = 0;
   double* d_tab = nullptr;
   float* d_tabf = nullptr;
@@ -123,7 +122,7 @@ static void free_ctx(mb_ctx* c) {
   if (c->gexec) cudaGraphExecDestroy(c->gexec);
   if (c->graph) cudaGraphDestroy(c->graph);
   void* ptrs[] = {c->d_blk, c->d_recmap, c->d_rec, c->d_grec, c->d_phys, c->d_cubic, c->d_cdst, c->d_csrc,
-                  c->d_pgsrc, c->d_tab, c->d_tabf, c->d_tab4, c->d_tab4f, c->d_st, c->d_tiles_sweep, c->d_tiles_aux, c->d_scratch, c->d_acc4, c->d_queue, c->d_recflux, c->d_brec, c->d_bcell,
+                  c->d_pgsrc, c->d_tab, c->d_tabf, c->d_tab4, c->d_tab4f, c->d_st, c->d_tiles_sweep, c->d_tiles_aux, c->d_scratch, c->d_acc4, c->d_queue, c->d_recflux, c->d_work,
                   c->d_physf, c->d_cubicf, c->d_tiles_km, c->d_irs, c->d_idst, c->d_isrc, c->d_ur, c->d_urb, c->d_dtl};
   for (void* q : ptrs)
     if (q) cudaFree(q);
@@ -332,14 +331,14 @@ static int check_mesh(const mb_mesh* mesh, int ngroups) {
 // frees the mesh-dependent device tables (blocks, record maps, records, ghost lists, tiles, FP32 geometry)
 static void free_tables(mb_ctx* c) {
   void* ptrs[] = {c->d_blk, c->d_recmap, c->d_rec, c->d_grec, c->d_phys, c->d_cubic, c->d_cdst, c->d_csrc,
-                  c->d_pgsrc, c->d_tiles_sweep, c->d_tiles_aux, c->d_recflux, c->d_brec, c->d_bcell,
+                  c->d_pgsrc, c->d_tiles_sweep, c->d_tiles_aux, c->d_recflux, c->d_work,
                   c->d_physf, c->d_cubicf, c->d_tiles_km, c->d_idst, c->d_isrc};
   for (void* q : ptrs)
     if (q) cudaFreeAsync(q, c->tstream);  // after the work queued on the table stream that may still read them
   c->d_idst = nullptr; c->d_isrc = nullptr;
   for (int d = 0; d < 4; ++d) c->irs_off[d] = 0;
   c->d_physf = nullptr; c->d_cubicf = nullptr; c->d_tiles_km = nullptr; c->ntiles_km = 0;
-  c->d_recflux = nullptr; c->d_brec = nullptr; c->d_bcell = nullptr; c->nrec = 0;
+  c->d_recflux = nullptr; c->d_work = nullptr; c->nrec = 0;
   c->d_blk = nullptr; c->d_recmap = nullptr; c->d_rec = nullptr; c->d_grec = nullptr; c->d_phys = nullptr;
   c->d_cubic = nullptr; c->d_cdst = nullptr; c->d_csrc = nullptr; c->d_pgsrc = nullptr;
   c->d_tiles_sweep = nullptr; c->d_tiles_aux = nullptr;
@@ -462,11 +461,10 @@ static int build_tables(mb_ctx* c, const mb_mesh* mesh) {
   for (int q = 0; q < mesh->nrec; ++q)
     if (!(hb[mesh->rec[q].blk].kmirror && mesh->rec[q].face >= 5) && mesh->rec[q].type != MB_BC_NONE) brec.push_back(q);
   std::stable_sort(brec.begin(), brec.end(), [&](int a, int b) { return mesh->rec[a].type < mesh->rec[b].type; });
-  std::vector<int> bcell(5 * brec.size());
+  std::vector<RecWork> work(brec.size());
   for (size_t q = 0; q < brec.size(); ++q) {
     const mb_bc& r = mesh->rec[brec[q]];
-    const int v[5] = {r.blk, r.i, r.j, r.k, r.face};
-    for (int a = 0; a < 5; ++a) bcell[5 * q + a] = v[a];
+    work[q] = RecWork{r.blk, r.i, r.j, r.k, r.face, r.type, brec[q], r.conn};
   }
   // ---- connections: ghost copies (2 layers) and the bc_pg source rows
   auto rowof = [&](int b, int i, int j, int k) -> long long {
@@ -640,8 +638,7 @@ static int build_tables(mb_ctx* c, const mb_mesh* mesh) {
   if ((rc = upload(&c->d_tiles_aux, ta.data(), ta.size(), c->tstream)) != MB_OK) return rc;
   if ((rc = upload(&c->d_tiles_km, tk.data(), tk.size(), c->tstream)) != MB_OK) return rc;
   c->ntiles_km = (int)tk.size();
-  if ((rc = upload(&c->d_brec, brec.data(), brec.size(), c->tstream)) != MB_OK) return rc;
-  if ((rc = upload(&c->d_bcell, bcell.data(), bcell.size(), c->tstream)) != MB_OK) return rc;
+  if ((rc = upload(&c->d_work, work.data(), work.size(), c->tstream)) != MB_OK) return rc;
   c->nrec = (int)brec.size();
   if (mesh->nrec > 0 &&
       cudaMallocAsync((void**)&c->d_recflux, (size_t)mesh->nrec * 2 * MB_NPRIM * sizeof(double), c->tstream) !=
@@ -1056,7 +1053,7 @@ static int records(mb_ctx* c, const double* Pin, cudaStream_t s) {
   if (c->nrec <= 0) return MB_OK;
   const Params& p = c->p;
   cudaError_t e;
-  e = MB_BY_FORM(c->sc.precision, sweep_unit(&c->sc), _records, (p, c->d_brec, c->d_bcell, c->nrec, Pin, s));
+  e = MB_BY_FORM(c->sc.precision, sweep_unit(&c->sc), _records, (p, c->d_work, c->nrec, Pin, s));
   c->launches += 1;
   CK(e);
   return MB_OK;

@@ -975,25 +975,50 @@ MB_HD void bc_record(const Params& p, const DBlk& b, const double* __restrict__ 
 }
 
 // Every boundary record of the mesh, one thread each, from the stage input P (ghosts filled): the contributions
-// (A, S) of record q go to recflux[q][0..9] in the flux type; the sweep adds them in face order after the interior
-// sum (BC_Fluxes after Fluxes, Mod_Explicit.f90:187-189).
+// (A, S) of record q go to recflux[q][0..9] in the flux type, or, on the simplified flux path of the solvers with their
+// own unit, the net one (A - S) to recflux[q][0..4]; the sweep adds them in face order after the interior sum
+// (BC_Fluxes after Fluxes, Mod_Explicit.f90:187-189). A warp's time is its chain of dependent loads, so what a record
+// needs to find its cells is one 32-byte entry (RecWork), and the connection records of that path take the interior
+// face's code and the FP32 geometry: one B200, a step with the records before and with them, 64 blocks of 32^3 mixed
+// 1572 and 1451 us, duct 121x67x45 430 and 399 us, 53^3 202 and 191 us.
 // VAR tells apart the instantiations of the same types built with different flags (the FP64 production form's units)
 template <typename R, bool VISC, int RS, int LIM, int VAR = 0>
-__global__ void __launch_bounds__(128) k_records(Params p, const int* __restrict__ brec, const int* __restrict__ bcell,
-                                               int nrec, const double* __restrict__ P) {
+__global__ void __launch_bounds__(128) k_records(Params p, const RecWork* __restrict__ work, int nrec,
+                                               const double* __restrict__ P) {
   pdl_next();
-  pdl_wait();
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
+  int4 w0 = make_int4(0, 0, 0, 0), w1 = w0;
+  if (q < nrec) {
+    w0 = __ldg(reinterpret_cast<const int4*>(work + q));
+    w1 = __ldg(reinterpret_cast<const int4*>(work + q) + 1);
+  }
+  pdl_wait();
   if (q >= nrec) return;
-  const int rid = brec[q];
-  const int* c = bcell + 5 * q;  // blk, i, j, k, face
-  const DBlk b = p.blk[c[0]];
+  const int rid = w1.z, face = w1.x, type = w1.y;
+  const DBlk& b = p.blk[w0.x];
   if (p.st[b.grp].done) return;
-  R v[2 * MB_NP];
-  bc_record<R, VISC, RS, LIM>(p, b, P, rid, c[1], c[2], c[3], c[4], v, v + MB_NP);
-  R* out = reinterpret_cast<R*>(p.recflux) + (long long)rid * 2 * MB_NP;
+  if constexpr (Fast<R>::on && RS != 0) {
+    R v[MB_NP];
+    if (type == 1) {
+      conn_fast<R, VISC, RS, LIM>(p, b, P, w0.y, w0.z, w0.w, face, p.pgsrc + (long long)w1.w * 6, v);
+    } else {
+      R S[MB_NP];
+      bc_record<R, VISC, RS, LIM>(p, b, P, rid, w0.y, w0.z, w0.w, face, v, S);
+      if (VISC) {
 #pragma unroll
-  for (int s = 0; s < 2 * MB_NP; ++s) out[s] = (VISC || s < MB_NP) ? v[s] : (R)0;
+        for (int s = 0; s < MB_NP; ++s) v[s] = v[s] - S[s];
+      }
+    }
+    R* out = reinterpret_cast<R*>(p.recflux) + (long long)rid * MB_NP;
+#pragma unroll
+    for (int s = 0; s < MB_NP; ++s) out[s] = v[s];
+  } else {
+    R v[2 * MB_NP];
+    bc_record<R, VISC, RS, LIM>(p, b, P, rid, w0.y, w0.z, w0.w, face, v, v + MB_NP);
+    R* out = reinterpret_cast<R*>(p.recflux) + (long long)rid * 2 * MB_NP;
+#pragma unroll
+    for (int s = 0; s < 2 * MB_NP; ++s) out[s] = (VISC || s < MB_NP) ? v[s] : (R)0;
+  }
 }
 
 // adds the record contributions of slot v (A = v[0..4], S = v[5..9]) into acc
@@ -1681,7 +1706,10 @@ __device__ __forceinline__ bool sweep_tile(const Params& p, const DTile t, const
         for (int F = 1; F <= nF; ++F) {
           if (!((on >> (F - 1)) & 1)) continue;
           const int rid = record_of(p, b, F, i, j, k);
-          if (rid >= 0) bc_apply<R, VISC>(rf + (long long)rid * 2 * MB_NP, acc);
+          if (rid >= 0) {
+            if constexpr (PAIR) bc_apply<R, false>(rf + (long long)rid * MB_NP, acc);
+            else bc_apply<R, VISC>(rf + (long long)rid * 2 * MB_NP, acc);
+          }
         }
         if (KM) {  // faces 5 and 6 of a mirrored block: the extrapolation records of every cell, computed here
           R A[MB_NP];

@@ -257,32 +257,21 @@ __device__ __forceinline__ void ausm_pair(const Params& p, const Side<R>& L, con
   fe = fp * h0L + fm * h0R;
 }
 
-// One interior face of direction d between cell (i,j,k) and its +d neighbour from the state tile: the net flux
-// (convective - viscous) into out[0..4]. (ii, jj): the tile coordinates of the cell.
-template <typename R, int TY, bool VISC, int RS, int LIM, bool KM, int NVT>
-__device__ __forceinline__ void face_fast(const Params& p, const DBlk& b, const Tile<R, TY, NVT, KM>& T, int d, int i,
-                                          int j, int k, int ii, int jj, R* out) {
-  constexpr int VS = Tile<R, TY, NVT, KM>::VS;
-  // the planes k-1 .. k+2 (a mirrored block's are its one plane)
-  const int S0 = slot_of<KM>(k - 1) * VS, S1 = slot_of<KM>(k) * VS, S2 = slot_of<KM>(k + 1) * VS,
-            S3 = slot_of<KM>(k + 2) * VS;
-  const int st = (d == 0) ? 1 : TXH;
-  const int o1 = jj * TXH + ii + S1;
-  const int o0 = o1 + ((d == 2) ? S0 - S1 : -st), o2 = o1 + ((d == 2) ? S2 - S1 : st),
-            o3 = o1 + ((d == 2) ? S3 - S1 : 2 * st);
-  const int l0 = lin32(b, i, j, k);
-  const int gst = (d == 0) ? 1 : (d == 1 ? b.pi : b.pi * b.pj);
+// The net flux (convective - viscous) along +d of the face between padded cell l0 of block b and its +d neighbour (gst
+// further on), into out[0..4]. c gives the states: c.stencil(q, A, B, C), q = 0..3, the four cells along d (1 and 2 the
+// face's own); c.transverse(e, w, A, B) the neighbours along the two other axes e in increasing order (w = 0, 1: below /
+// above cell 1; 2, 3: below / above cell 2).
+template <typename R, bool VISC, int RS, int LIM, typename Cells>
+__device__ __forceinline__ void face_core(const Params& p, const DBlk& b, int d, int l0, int gst, int face,
+                                          const Cells& c, R* out) {
   R nx, ny, nz, area;
-  face_rec(b, d, fmi32(b, d, i, j, k), nx, ny, nz, area);
+  face_rec(b, d, face, nx, ny, nz, area);
   if (nx == (R)0 && ny == (R)0 && nz == (R)0) area = (R)0;  // a degenerate face carries no flux
   // ---- the viscous flux first (its four values are fewer to keep than the face's two cells)
   V2<R> vuv;
   R vw, ve;
   R dl1, dl2;
   if (VISC) {
-    // the transverse neighbours: cells -/+ along the axes b and c of both cells (b, c in increasing order)
-    const int sb = (d == 0) ? TXH : 1;
-    const int cm = (d == 2) ? -TXH : S0 - S1, cq = (d == 2) ? TXH : S2 - S1;
     V2<R> GnA, GnB, Gt;  // grad(.) . n of (u, v), (w, T); (grad u)^T n, x and y
     R Gtz, div;
     auto add_axis = [&](const V2<R>& gA, const V2<R>& gB, const V2<R>& m, R z, bool first) {
@@ -301,12 +290,12 @@ __device__ __forceinline__ void face_fast(const Params& p, const DBlk& b, const 
     const int ab = (d == 0) ? 1 : 0, ac = (d == 2) ? 1 : 2;
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
-      const int lo_ = e ? cm : -sb, hi_ = e ? cq : sb, ax = e ? ac : ab;
+      const int ax = e ? ac : ab;
       V2<R> a0, b0, a1, b1, a2, b2, a3, b3;
-      T.load_uvwT(o1 + lo_, a0, b0);
-      T.load_uvwT(o1 + hi_, a1, b1);
-      T.load_uvwT(o2 + lo_, a2, b2);
-      T.load_uvwT(o2 + hi_, a3, b3);
+      c.transverse(e, 0, a0, b0);
+      c.transverse(e, 1, a1, b1);
+      c.transverse(e, 2, a2, b2);
+      c.transverse(e, 3, a3, b3);
       V2<R> m, m2;
       R z, z2, dd;
       metric(b, ax, l0, m, z, dd);
@@ -315,8 +304,8 @@ __device__ __forceinline__ void face_fast(const Params& p, const DBlk& b, const 
     }
     V2<R> A1, B1, C1, A2, B2, C2, m, m2;
     R z, z2;
-    T.load(o1, A1, B1, C1);
-    T.load(o2, A2, B2, C2);
+    c.stencil(1, A1, B1, C1);
+    c.stencil(2, A2, B2, C2);
     metric(b, d, l0, m, z, dl1);
     metric(b, d, l0 + gst, m2, z2, dl2);
     const V2<R> four = dup2<R>((R)4);
@@ -344,21 +333,21 @@ __device__ __forceinline__ void face_fast(const Params& p, const DBlk& b, const 
     const V2<R> I0 = dup2<R>(i0), I1 = dup2<R>(i1), I2 = dup2<R>(i2), LM = dup2<R>((R)0.5 * dl1),
                 LP = dup2<R>((R)-0.5 * dl2);
     auto face_states = [&](const V2<R>& q0, const V2<R>& q1, const V2<R>& q2, const V2<R>& q3, V2<R>& l, V2<R>& r) {
-      const V2<R> a = (q1 - q0) * I0, e = (q2 - q1) * I1, c = (q3 - q2) * I2;
+      const V2<R> a = (q1 - q0) * I0, e = (q2 - q1) * I1, f = (q3 - q2) * I2;
       V2<R> sl, sr;
       if (LIM == 3) {
-        sl = albada(a, e, c, sr);
+        sl = albada(a, e, f, sr);
       } else {
         const int lim = LIM ? LIM : p.lim;
         sl = mk2<R>(slope_rt<R>(lim, lo2(e), lo2(a)), slope_rt<R>(lim, hi2(e), hi2(a)));
-        sr = mk2<R>(slope_rt<R>(lim, lo2(c), lo2(e)), slope_rt<R>(lim, hi2(c), hi2(e)));
+        sr = mk2<R>(slope_rt<R>(lim, lo2(f), lo2(e)), slope_rt<R>(lim, hi2(f), hi2(e)));
       }
       l = fma2(sl, LM, q1);
       r = fma2(sr, LP, q2);
     };
     V2<R> A[4], B[4], C[4], l, r;
 #pragma unroll
-    for (int q = 0; q < 4; ++q) T.load(q == 0 ? o0 : q == 1 ? o1 : q == 2 ? o2 : o3, A[q], B[q], C[q]);
+    for (int q = 0; q < 4; ++q) c.stencil(q, A[q], B[q], C[q]);
     face_states(A[0], A[1], A[2], A[3], L.A, Q.A);
     face_states(B[0], B[1], B[2], B[3], l, r);
     L.w = lo2(l); Q.w = lo2(r);
@@ -384,6 +373,86 @@ __device__ __forceinline__ void face_fast(const Params& p, const DBlk& b, const 
   out[MB_IV] = hi2(F);
   out[MB_IW] = fw * area;
   out[MB_IPR] = fe * area;
+}
+
+// the cells of an interior face in the state tile
+template <typename R, int TY, bool KM, int NVT>
+struct TileCells {
+  const Tile<R, TY, NVT, KM>& T;
+  int o0, o1, o2, o3;  // the stencil
+  int bm, cm, cp;      // offsets below / above along the two transverse axes: -bm, bm; cm, cp
+  __device__ __forceinline__ void stencil(int q, V2<R>& A, V2<R>& B, V2<R>& C) const {
+    T.load(q == 0 ? o0 : q == 1 ? o1 : q == 2 ? o2 : o3, A, B, C);
+  }
+  __device__ __forceinline__ void transverse(int e, int w, V2<R>& A, V2<R>& B) const {
+    T.load_uvwT((w < 2 ? o1 : o2) + (e == 0 ? ((w & 1) ? bm : -bm) : ((w & 1) ? cp : cm)), A, B);
+  }
+};
+
+// One interior face of direction d between cell (i,j,k) and its +d neighbour from the state tile; (ii, jj): the tile
+// coordinates of the cell
+template <typename R, int TY, bool VISC, int RS, int LIM, bool KM, int NVT>
+__device__ __forceinline__ void face_fast(const Params& p, const DBlk& b, const Tile<R, TY, NVT, KM>& T, int d, int i,
+                                          int j, int k, int ii, int jj, R* out) {
+  constexpr int VS = Tile<R, TY, NVT, KM>::VS;
+  // the planes k-1 .. k+2 (a mirrored block's are its one plane)
+  const int S0 = slot_of<KM>(k - 1) * VS, S1 = slot_of<KM>(k) * VS, S2 = slot_of<KM>(k + 1) * VS,
+            S3 = slot_of<KM>(k + 2) * VS;
+  const int st = (d == 0) ? 1 : TXH;
+  const int o1 = jj * TXH + ii + S1;
+  const TileCells<R, TY, KM, NVT> c{T, o1 + ((d == 2) ? S0 - S1 : -st), o1, o1 + ((d == 2) ? S2 - S1 : st),
+                                    o1 + ((d == 2) ? S3 - S1 : 2 * st), (d == 0) ? TXH : 1,
+                                    (d == 2) ? -TXH : S0 - S1, (d == 2) ? TXH : S2 - S1};
+  face_core<R, VISC, RS, LIM>(p, b, d, lin32(b, i, j, k), (d == 0) ? 1 : (d == 1 ? b.pi : b.pi * b.pj),
+                              fmi32(b, d, i, j, k), c, out);
+}
+
+// the cells of a connection record's face in the state arena: the boundary cell and the ghosts of its face, filled; the
+// ghost's transverse neighbours are the donor's (the rows pg[2..5] of the record's table: -b, +b, -c, +c)
+template <typename R>
+struct ArenaCells {
+  const double* P;
+  long long nc, row1, st;  // row1: the lower cell of the face
+  long long own, sb, sc;   // the boundary cell's row and its transverse strides
+  const long long* pg;
+  R iri;
+  bool low;                // the boundary cell is the upper one (a low face)
+  __device__ __forceinline__ void uvwT(long long r, V2<R>& A, V2<R>& B, V2<R>& C) const {
+    const R rho = (R)ld(P + r), u = (R)ld(P + r + nc), v = (R)ld(P + r + 2 * nc), w = (R)ld(P + r + 3 * nc),
+            pr = (R)ld(P + r + 4 * nc);
+    A = mk2<R>(u, v);
+    B = mk2<R>(w, pr * iri * rcp_(rho));
+    C = mk2<R>(rho, pr);
+  }
+  __device__ __forceinline__ void stencil(int q, V2<R>& A, V2<R>& B, V2<R>& C) const { uvwT(row1 + (q - 1) * st, A, B, C); }
+  __device__ __forceinline__ void transverse(int e, int w, V2<R>& A, V2<R>& B) const {
+    const bool mine = (w >= 2) == low;
+    const long long s = e == 0 ? sb : sc;
+    const long long r = mine ? own + ((w & 1) ? s : -s) : ld_row(pg + 2 + 2 * e + (w & 1));
+    V2<R> C;
+    uvwT(r, A, B, C);
+  }
+  __device__ __forceinline__ static long long ld_row(const long long* q) { return __ldg(q); }
+};
+
+// a connection record (bc_conn_eul and bc_conn_visc of mb_engine.cuh): the net contribution to the row of its cell. The
+// two viscous fluxes the reference averages, with the gradients of the cell and of its ghost, are one flux with the
+// mean gradient (the flux is linear in it): the interior face's.
+template <typename R, bool VISC, int RS, int LIM>
+__device__ __forceinline__ void conn_fast(const Params& p, const DBlk& b, const double* __restrict__ P, int i, int j,
+                                          int k, int F, const long long* __restrict__ pg, R* out) {
+  const int d = (F - 1) >> 1, low = F & 1;
+  const int gst = (d == 0) ? 1 : (d == 1 ? b.pi : b.pi * b.pj);
+  const int l = lin32(b, i, j, k);
+  const int il = (d == 0) ? i - low : i, jl = (d == 1) ? j - low : j, kl = (d == 2) ? k - low : k;
+  const int sk = b.kmirror ? 0 : b.pi * b.pj;  // a mirrored block's k ghosts are its k = 1 cells
+  const ArenaCells<R> c{P, p.nc, b.boff + l - low * gst, gst, b.boff + l, (d == 0) ? b.pi : 1, (d == 2) ? b.pi : sk, pg,
+                        Cst<R>::of(p).iri, low != 0};
+  face_core<R, VISC, RS, LIM>(p, b, d, l - low * gst, gst, fmi32(b, d, il, jl, kl), c, out);
+  if (low) {
+#pragma unroll
+    for (int s = 0; s < MB_NP; ++s) out[s] = -out[s];
+  }
 }
 
 }  // namespace mb

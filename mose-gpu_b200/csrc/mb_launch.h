@@ -68,8 +68,7 @@ static inline cudaError_t launch_chained(bool chain, void (*kernel)(K...), unsig
   cudaError_t name(const Params& p, const DTile* tiles, int ntiles, int mode, const double* Pin, const double* Pold, \
                    double* Pout, double* Rout, double rkc, int last, int km, cudaStream_t s);                      \
   cudaError_t name##_setup();                                                                                    \
-  cudaError_t name##_records(const Params& p, const int* brec, const int* bcell, int nrec, const double* P,      \
-                             cudaStream_t s);                                                                    \
+  cudaError_t name##_records(const Params& p, const RecWork* work, int nrec, const double* P, cudaStream_t s);   \
   cudaError_t name##_dt(const Params& p, const DTile* tiles, int ntiles, const double* P, int only_group,       \
                         cudaStream_t s);                                                                         \
   int name##_occupancy(int visc, int lim);                                                                       \

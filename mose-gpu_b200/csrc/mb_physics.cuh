@@ -89,6 +89,13 @@ struct DRec {
   double q[16];
 };
 
+// the record kernel's work entry: where the record's cell is, its face and type, its index and, for a connection, its
+// row of the transverse-stencil table
+struct __align__(16) RecWork {
+  int blk, i, j, k;
+  int face, type, rec, pg;
+};
+
 // device status + clock of the time loop (one per context)
 struct DevState {
   unsigned long long dtmin_bits;  // min of the local dt of the step being computed (positive doubles order as u64)
