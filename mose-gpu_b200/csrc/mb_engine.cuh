@@ -1517,7 +1517,8 @@ __device__ __forceinline__ void stage_plane_raw(const Params& p, const DBlk& b, 
 template <typename R, int TY, bool VISC, int MODE, int RS, int LIM, bool KM, int STG>
 __device__ __forceinline__ bool sweep_tile(const Params& p, const DTile t, const double* __restrict__ Pin,
                                            const double* Pold, double* Pout, double* Rout, double rkc, int last,
-                                           unsigned char* smem_raw, double* sred, double* s_res, TmaStage& ts) {
+                                           unsigned char* smem_raw, double* sred, double* s_res, TmaStage& ts,
+                                           DBlk& sblk) {
   unsigned char* raw = ts.halo;
   unsigned long long* bar = ts.bar_halo;
   unsigned& phase = ts.ph_halo;
@@ -1546,7 +1547,13 @@ __device__ __forceinline__ bool sweep_tile(const Params& p, const DTile t, const
   R kup[NS], kdn[NS];
 #pragma unroll
   for (int q = 0; q < NS; ++q) kup[q] = kdn[q] = (R)0;
-  const DBlk b = p.blk[t.blk];
+  // the block in shared memory: a local copy went to the stack (its record maps are indexed at run time), and its fields
+  // came back through local loads. A step with the stack copy and so: 2-D batch 693 and 588 us, 16 served cases 3.04 and
+  // 2.59 ms, 192^3 mixed 3.11 and 3.07 ms.
+  for (int w = threadIdx.x; w < (int)(sizeof(DBlk) / 4); w += blockDim.x)
+    reinterpret_cast<int*>(&sblk)[w] = __ldg(reinterpret_cast<const int*>(p.blk + t.blk) + w);
+  __syncthreads();
+  const DBlk& b = sblk;
   DevState* st = p.st + b.grp;
   if (MODE == MODE_UPDATE && st->done) return true;  // the case has reached its stop time (uniform over the CTA)
   // TMA staging (uniform over the CTA; without a map the TMA form stages the same tile values by plain loads)
@@ -1587,7 +1594,7 @@ __device__ __forceinline__ bool sweep_tile(const Params& p, const DTile t, const
   // the first plane of the loop in flight while the k-face below is computed
   if (tma && t.k0 + 2 <= b.n3 + kext) tma_issue_plane<TY>(p, b, raw, bar, t.i0, t.j0, t.k0 + 2);
   __syncthreads();
-  if (own && t.k0 > 1) {
+  if (!KM && own && t.k0 > 1) {
     R out[NF];
     if constexpr (PAIR) face_fast<R, TY, VISC, RS, LIM, KM, NVT>(p, b, T, 2, i, j, t.k0 - 1, tx + 2, ty + 2, out);
     else face_flux<R, TY, VISC, RS, LIM, KM, NVT>(p, b, T, 2, i, j, t.k0 - 1, tx + 2, ty + 2, out);
@@ -1621,6 +1628,45 @@ __device__ __forceinline__ bool sweep_tile(const Params& p, const DTile t, const
     if (tma && k + 3 <= b.n3 + kext && k + 1 < t.k1) tma_issue_plane<TY>(p, b, raw, bar, t.i0, t.j0, k + 3);
     // ---- face tasks of this plane through one call site: 0 = i-face #tid, 1 = extra i-faces (last warp,
     // lanes < TY), 2 = j-face #tid, 3 = extra j-face row (warp 0), 4 = the k-face above
+    if constexpr (PAIR) {
+      // one call site per direction: with a literal d the offsets and pointers need no selects, and the shorter face code
+      // no longer crowds the instruction cache. One B200, a step with one call site for all and so: 192^3 mixed 3.06 and
+      // 2.95 ms, the 12-block 2-D batch 577 and 527 us, eight steps of 2-D 301^2 707 and 662 us.
+#pragma unroll 1
+      for (int rep = 0; rep < 2; ++rep) {  // i-faces
+        if (rep == 1 && (ty != TY - 1 || tx >= TY)) break;
+        const int f = rep == 0 ? tid : 32 * TY + tx;
+        const int rw = f / 33, cl = f - rw * 33;
+        const int fi = t.i0 + cl - 1, fj = t.j0 + rw;
+        if (fi >= 1 && fi <= b.n1 - 1 && fj <= b.n2) {
+          R out[NF];
+          face_fast<R, TY, VISC, RS, LIM, KM, NVT>(p, b, T, 0, fi, fj, k, cl + 1, rw + 2, out);
+#pragma unroll
+          for (int q = 0; q < NS; ++q) sFi[rw][cl][q] = out[q];
+        }
+      }
+#pragma unroll 1
+      for (int rep = 0; rep < 2; ++rep) {  // j-faces
+        if (rep == 1 && ty != 0) break;
+        const int rw = rep == 0 ? ty : TY;
+        const int fi = t.i0 + tx, fj = t.j0 + rw - 1;
+        if (fj >= 1 && fj <= b.n2 - 1 && fi <= b.n1) {
+          R out[NF];
+          face_fast<R, TY, VISC, RS, LIM, KM, NVT>(p, b, T, 1, fi, fj, k, tx + 2, rw + 1, out);
+#pragma unroll
+          for (int q = 0; q < NS; ++q) sFj[rw][tx][q] = out[q];
+        }
+      }
+      if (!KM && own && k < b.n3) {  // the k-face above
+        R out[NF];
+        face_fast<R, TY, VISC, RS, LIM, KM, NVT>(p, b, T, 2, i, j, k, tx + 2, ty + 2, out);
+#pragma unroll
+        for (int q = 0; q < NS; ++q) {
+          if (KREG) kup[q] = out[q];
+          else sFk0[kb * TY + ty][tx][q] = out[q];
+        }
+      }
+    } else {
 #pragma unroll 1
     for (int task = 0; task < 5; ++task) {
       int d = -1, fi = 0, fj = 0, ii = 0, jj = 0;
@@ -1654,6 +1700,7 @@ __device__ __forceinline__ bool sweep_tile(const Params& p, const DTile t, const
 #pragma unroll
         for (int q = 0; q < NS; ++q) dst[q] = NET ? out[q] - out[MB_NP + q] : out[q];
       }
+    }
     }
     __syncthreads();
     // the residual diagnostic of the last stage: (new - old)^2 of this thread's cell, in the flux type (the warps'
@@ -1826,6 +1873,7 @@ k_sweep(Params p, const DTile* __restrict__ tiles, const double* __restrict__ Pi
   __shared__ double sred[32];
   __shared__ double s_res[8 * MB_NP];  // per warp (at most 8) and variable: the tile's residual sums
   __shared__ int s_next;
+  __shared__ DBlk s_blk;
   __shared__ __align__(8) unsigned long long s_bar;  // TMA staging: the mbarrier of the landing plane
   static_assert(TY <= 8, "one residual slot per warp");
   pdl_next();
@@ -1845,7 +1893,7 @@ k_sweep(Params p, const DTile* __restrict__ tiles, const double* __restrict__ Pi
   pdl_wait();
   if (!p.queue) {
     sweep_tile<R, TY, VISC, MODE, RS, LIM, KM, STG>(p, tiles[blockIdx.x], Pin, Pold, Pout, Rout, rkc, last, smem_raw,
-                                                     sred, s_res, ts);
+                                                     sred, s_res, ts, s_blk);
     return;
   }
   for (;;) {
@@ -1854,7 +1902,7 @@ k_sweep(Params p, const DTile* __restrict__ tiles, const double* __restrict__ Pi
     const int tix = s_next;
     if (tix >= p.ntiles_run) break;
     if (!sweep_tile<R, TY, VISC, MODE, RS, LIM, KM, STG>(p, tiles[tix], Pin, Pold, Pout, Rout, rkc, last, smem_raw,
-                                                          sred, s_res, ts))
+                                                          sred, s_res, ts, s_blk))
       break;
     __syncthreads();  // the tile's shared memory is free and s_next may be overwritten
   }
