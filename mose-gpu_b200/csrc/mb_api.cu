@@ -739,7 +739,7 @@ int mb_init(const mb_mesh* mesh, const mb_scheme* sc, const mb_thermo* th, int d
   c->sc = *sc;
   c->ncell = mesh->ncell_total;
   c->ngroups = ngroups;
-  c->ty_sweep = sc->precision == MB_PREC_MIXED ? TY_F32 : TY_F64;
+  c->ty_sweep = sc->precision == MB_PREC_MIXED ? TY_F32 : (sc->precision == MB_PREC_FP64_FAST ? TY_F64F : TY_F64);
   c->no_tma = getenv("MB_NO_TMA") != nullptr;
 #define TRY(x)                 \
   do {                         \

@@ -35,7 +35,10 @@ struct GhostLists {
   int cubic_off[3];
 };
 
-constexpr int TY_F64 = 4;    // tile rows of the FP64 sweep (128 threads)
+constexpr int TY_F64 = 4;    // tile rows of the FP64 parity sweep (128 threads)
+constexpr int TY_F64F = 6;   // tile rows of the FP64 production sweep: 192 threads at 168 registers, 12 warps per SM and
+                             // fewer j-faces computed twice than 4 rows (128 threads, 232 registers, 8 warps per SM):
+                             // a step of 96^3 1.71 and 1.45 ms, of the 4-block 2-D batch 370 and 312 us
 constexpr int TY_F32 = 8;    // tile rows of the mixed sweep (256 threads)
 constexpr int MINB_F64 = 2;  // resident CTAs per SM the FP64 sweep's registers must allow
 constexpr int MINB_F32 = 3;  // resident CTAs per SM the mixed sweep's registers must allow (80 registers)
