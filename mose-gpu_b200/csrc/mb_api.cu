@@ -655,6 +655,14 @@ static int build_tables(mb_ctx* c, const mb_mesh* mesh) {
   g.cdst = c->d_cdst; g.csrc = c->d_csrc; g.ncopy = (int)cdst.size(); g.pgsrc = c->d_pgsrc; g.nconn = mesh->nconn;
   g.ordered = ordered;
   g.fused = !ordered && deep_donors;
+  bool reads_ghosts = false;  // a record of the work list reads a ghost row
+  for (const RecWork& w : work) {
+    const int ax = (w.face - 1) / 2;
+    if (w.type == MB_BC_CONNECTION || (w.type == MB_BC_SYMMETRY && sc->visc) ||
+        (w.type != MB_BC_EXTRAPOLATION && mesh->blk[w.blk].n[ax] < 2))
+      reads_ghosts = true;
+  }
+  g.surface = g.fused && !reads_ghosts && sc->intvar != 2;
   for (int f = 0; f < 3; ++f) { g.phys_off[f] = po[f]; g.cubic_off[f] = co[f]; }
   c->gf = g;
   c->gf.phys = c->d_physf; c->gf.nphys = (int)physf.size(); c->gf.cubic = c->d_cubicf; c->gf.ncubic = (int)cubicf.size();
@@ -1049,11 +1057,19 @@ static int sweep_on(mb_ctx* c, const DTile* t, int n, int persistent, int mode, 
 }
 
 // the boundary records of the stage input (BC_Fluxes), before the sweep that adds them
-static int records(mb_ctx* c, const double* Pin, cudaStream_t s) {
-  if (c->nrec <= 0) return MB_OK;
+// (surface: with the stage's ghost fill and, on clock, the case clocks in the same launch)
+static int records(mb_ctx* c, const double* Pin, cudaStream_t s, bool surface = false, bool clock = false) {
+  Surface sf{};
+  if (surface) {
+    sf.grec = c->gf.rec; sf.phys = c->gf.phys; sf.P = const_cast<double*>(Pin);
+    sf.nphys = c->gf.nphys;
+    sf.nblk_ghost = (sf.nphys + 127) / 128;
+    sf.clock = clock ? 1 : 0;
+  }
+  if (c->nrec + sf.nblk_ghost + sf.clock <= 0) return MB_OK;
   const Params& p = c->p;
   cudaError_t e;
-  e = MB_BY_FORM(c->sc.precision, sweep_unit(&c->sc), _records, (p, c->d_work, c->nrec, Pin, s));
+  e = MB_BY_FORM(c->sc.precision, sweep_unit(&c->sc), _records, (p, c->d_work, c->nrec, Pin, sf, s));
   c->launches += 1;
   CK(e);
   return MB_OK;
@@ -1095,9 +1111,9 @@ static int time_sweep(mb_ctx* c, const std::vector<DTile>& tl, int persistent, c
   return rc;
 }
 
-static int fill(mb_ctx* c, double* P, cudaStream_t s, bool fused = true) {
+static int fill(mb_ctx* c, double* P, cudaStream_t s, bool fused = true, bool clock = false) {
   int nl = 0;
-  cudaError_t e = ghost_fill(c->p, fused ? c->gf : c->g, P, s, &nl);
+  cudaError_t e = ghost_fill(c->p, fused ? c->gf : c->g, P, s, &nl, clock);
   c->launches += nl;
   CK(e);
   return MB_OK;
@@ -1276,7 +1292,11 @@ static int stage_compute(mb_ctx* c, const double* in, const double* P, double* o
   return MB_OK;
 }
 
-static int stage(mb_ctx* c, double* P, double* PO, int irk, cudaStream_t s) {
+// the clock of a step can be advanced by the first stage's ghost fill: nothing in that launch reads it
+static bool clock_in_fill(const mb_ctx* c) { return c->gf.fused && !c->p.prec; }
+
+// clock: the stage also advances the case clocks, before its sweep (only where clock_in_fill)
+static int stage(mb_ctx* c, double* P, double* PO, int irk, cudaStream_t s, bool clock = false) {
   const int n = c->sc.n_rk;
   double* S = c->d_scratch;
   const double* in;
@@ -1284,9 +1304,12 @@ static int stage(mb_ctx* c, double* P, double* PO, int irk, cudaStream_t s) {
   stage_buffers(n, irk, P, PO, S, &in, &outp);
   int rc = ur_pass(c, in, s);  // prec: Ur of the stage input
   if (rc != MB_OK) return rc;
-  rc = fill(c, const_cast<double*>(in), s);
-  if (rc != MB_OK) return rc;
-  rc = records(c, in, s);
+  const bool surface = c->gf.surface;
+  if (!surface) {
+    rc = fill(c, const_cast<double*>(in), s, true, clock);
+    if (rc != MB_OK) return rc;
+  }
+  rc = records(c, in, s, surface, surface && clock);
   if (rc != MB_OK) return rc;
   const int last = (irk == n) ? 1 : 0;
   rc = stage_compute(c, in, P, outp, irk, last, s);
@@ -1439,10 +1462,13 @@ static int one_step(mb_ctx* c, double* P, double* PO, cudaStream_t s) {
     int rc = dt_min(c, P, s);
     if (rc != MB_OK) return rc;
   }
-  CK(clock_step(c->p, s));
-  c->launches += 1;
+  const bool ck = clock_in_fill(c);
+  if (!ck) {
+    CK(clock_step(c->p, s));
+    c->launches += 1;
+  }
   for (int irk = 1; irk <= c->sc.n_rk; ++irk) {
-    int rc = stage(c, P, PO, irk, s);
+    int rc = stage(c, P, PO, irk, s, ck && irk == 1);
     if (rc != MB_OK) return rc;
   }
   return MB_OK;

@@ -974,6 +974,97 @@ MB_HD void bc_record(const Params& p, const DBlk& b, const double* __restrict__ 
   }
 }
 
+// ---- the ghosts of one record and the case clocks, in explicitly rounded operations: the same bits in every unit
+// (Fill_Ghost_Cell_blk, Lib_Extrapolation.f90:643-730, and the cubic ghosts :859-879; see mb_f64.cu)
+struct GRec {
+  int blk, i, j, k, face, type;
+};
+
+// the surface work that shares the record kernel's launch (nblk_ghost, clock: blocks after the records' ones)
+struct Surface {
+  const GRec* grec;
+  const int* phys;
+  double* P;
+  int nphys, nblk_ghost, clock;
+};
+
+__device__ __forceinline__ double cubic_ghost(double a1, double a2, double a3) {
+  return __dadd_rn(__dsub_rn(__dmul_rn(3.0, a1), __dmul_rn(3.0, a2)), a3);
+}
+
+// entry e: the record and in bits 28-29 its layer count (0: both); no ghost is computed from another one's (fused lists)
+__device__ __forceinline__ void ghost_record(const Params& p, const GRec* __restrict__ rec, int e, double* P) {
+  const int nl = (e >> 28) ? (e >> 28) : GC;
+  const GRec r = rec[e & 0x0fffffff];
+  const DBlk& b = p.blk[r.blk];
+  const long long nc = p.nc;
+  const int dir = (r.face + 1) / 2, step = 1 - 2 * (r.face % 2);  // away from the block
+  const long long st = step * ((dir == 1) ? 1 : (dir == 2 ? (long long)b.pi : (long long)b.pi * b.pj));
+  const long long c = row(b, r.i, r.j, r.k);
+  if (r.type == 3) {  // Ghost_Symmetry: the first layer, normal velocity reversed
+    double g[4];
+    bc_face_geom(b, r.i, r.j, r.k, r.face, g);
+    double vel[3] = {P[c + MB_IU * nc], P[c + MB_IV * nc], P[c + MB_IW * nc]};
+    const double udotn = __dadd_rn(__dadd_rn(__dmul_rn(vel[0], g[0]), __dmul_rn(vel[1], g[1])), __dmul_rn(vel[2], g[2]));
+    for (int a = 0; a < 3; ++a) vel[a] = __dsub_rn(vel[a], __dmul_rn(2.0 * udotn, g[a]));
+    P[c + st] = P[c];
+    P[c + st + MB_IU * nc] = vel[0]; P[c + st + MB_IV * nc] = vel[1]; P[c + st + MB_IW * nc] = vel[2];
+    P[c + st + MB_IPR * nc] = P[c + MB_IPR * nc];
+    return;
+  }
+  const int nax = dir == 1 ? b.n1 : (dir == 2 ? b.n2 : b.n3);
+  const bool cubic = r.type == 5 || r.type == 6 || (r.type == 11 && nax > 1);
+#pragma unroll
+  for (int s = 0; s < MB_NP; ++s) {
+    double* q0 = P + c + s * nc;
+    const double a1 = q0[0];
+    if (cubic) {  // 3 x1 - 3 x2 + x3, the second layer from the first
+      const double a2 = q0[-st], g1 = cubic_ghost(a1, a2, q0[-2 * st]);
+      q0[st] = g1;
+      if (nl > 1) q0[2 * st] = cubic_ghost(g1, a1, a2);
+    } else {
+      q0[st] = a1;
+      if (nl > 1) q0[2 * st] = a1;
+    }
+  }
+}
+
+// the step's dt of every case (Compute_dt's dtglobal = 1e5 then the cell minimum, Mod_Explicit.f90:122;
+// Set_Global_dt; Clip_dt_To_Timemax, Mod_dt.f90:283-296), its simulated time, and a fresh minimum for the
+// next step. A case whose time has reached its stop time (the reference's time-loop exit) is marked done and
+// no longer advances.
+__device__ __forceinline__ void clock_groups(const Params& p) {
+  for (int g = threadIdx.x; g < p.ngroups; g += blockDim.x) {
+    DevState* st = p.st + g;
+    if (st->done) continue;
+    if (st->t_end > 0.0 && st->time >= st->t_end) {
+      st->done = 1;
+      continue;
+    }
+    // the residual end test of the step just taken (Mod_Explicit.f90:363-370: residuotot(1) <= restop)
+    if (st->res_stop > 0.0 && st->steps > 0 && sqrt(st->res2[0]) <= st->res_stop) {
+      st->done = 1;
+      continue;
+    }
+    // cfl-rise-threshold: the factor of step iter (Mod_dt.f90:57-58); the minimum of the scaled local steps is the
+    // scaled minimum (a product with a positive factor rounds monotonically)
+    const int iter = st->steps + 1;
+    st->rampf = (iter < p.cfl_rise) ? (double)iter / p.cfl_rise : 1.0;
+    double dtg = 1e5;
+    double dm = __longlong_as_double((long long)st->dtmin_bits);
+    dtg = mn(__dmul_rn(dm, st->rampf), dtg);
+    if (st->time_clip && !p.local_dt) {
+      double rem = st->t_end - st->time;
+      if (rem > 0.0 && dtg > rem) dtg = __dmul_rn(rem, 1.0 + 1e-12);
+    }
+    st->dt = dtg;
+    if (!p.local_dt) st->time = __dadd_rn(st->time, dtg);  // time-accurate = false: no time (Mod_Explicit.f90:124-128)
+    st->steps = st->steps + 1;
+    st->dtmin_bits = (unsigned long long)__double_as_longlong(1e300);
+    for (int v = 0; v < MB_NP; ++v) st->res2[v] = 0.0;
+  }
+}
+
 // Every boundary record of the mesh, one thread each, from the stage input P (ghosts filled): the contributions
 // (A, S) of record q go to recflux[q][0..9] in the flux type, or, on the simplified flux path of the solvers with their
 // own unit, the net one (A - S) to recflux[q][0..4]; the sweep adds them in face order after the interior sum
@@ -984,8 +1075,16 @@ MB_HD void bc_record(const Params& p, const DBlk& b, const double* __restrict__ 
 // VAR tells apart the instantiations of the same types built with different flags (the FP64 production form's units)
 template <typename R, bool VISC, int RS, int LIM, int VAR = 0>
 __global__ void __launch_bounds__(128) k_records(Params p, const RecWork* __restrict__ work, int nrec,
-                                               const double* __restrict__ P) {
+                                               const double* __restrict__ P, Surface sf) {
   pdl_next();
+  const int nbr = (nrec + 127) / 128;
+  if ((int)blockIdx.x >= nbr) {  // the ghosts and the clock (meshes whose records read no ghost)
+    pdl_wait();
+    const int g = (blockIdx.x - nbr) * blockDim.x + threadIdx.x;
+    if ((int)blockIdx.x - nbr >= sf.nblk_ghost) clock_groups(p);
+    else if (g < sf.nphys) ghost_record(p, sf.grec, sf.phys[g], sf.P);
+    return;
+  }
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
   int4 w0 = make_int4(0, 0, 0, 0), w1 = w0;
   if (q < nrec) {

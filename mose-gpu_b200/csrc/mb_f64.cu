@@ -52,9 +52,14 @@ __global__ void k_ghost_phys(Params p, const GRec* __restrict__ rec, const int* 
 // one.
 __global__ void __launch_bounds__(128) k_ghost_fill(Params p, const GRec* __restrict__ rec, const int* __restrict__ list,
                                                     int n, int nblk_rec, const long long* __restrict__ dst,
-                                                    const long long* __restrict__ src, int ncopy, double* P) {
+                                                    const long long* __restrict__ src, int ncopy, double* P,
+                                                    int clock) {
   pdl_next();
   pdl_wait();
+  if (clock && blockIdx.x == gridDim.x - 1) {
+    clock_groups(p);
+    return;
+  }
   const long long nc = p.nc;
   if ((int)blockIdx.x >= nblk_rec) {
     const int e = (blockIdx.x - nblk_rec) * blockDim.x + threadIdx.x;  // one thread per row: its five variables
@@ -69,41 +74,7 @@ __global__ void __launch_bounds__(128) k_ghost_fill(Params p, const GRec* __rest
     return;
   }
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= n) return;
-  const int e = list[q];
-  const int nl = (e >> 28) ? (e >> 28) : GC;
-  const GRec r = rec[e & 0x0fffffff];
-  const DBlk& b = p.blk[r.blk];
-  const int dir = (r.face + 1) / 2, step = 1 - 2 * (r.face % 2);  // away from the block
-  const long long st = step * ((dir == 1) ? 1 : (dir == 2 ? (long long)b.pi : (long long)b.pi * b.pj));
-  const long long c = row(b, r.i, r.j, r.k);
-  if (r.type == 3) {  // Ghost_Symmetry: the first layer, normal velocity reversed
-    double g[4];
-    bc_face_geom(b, r.i, r.j, r.k, r.face, g);
-    double vel[3] = {P[c + MB_IU * nc], P[c + MB_IV * nc], P[c + MB_IW * nc]};
-    const double udotn = vel[0] * g[0] + vel[1] * g[1] + vel[2] * g[2];
-    for (int a = 0; a < 3; ++a) vel[a] = vel[a] - 2.0 * udotn * g[a];
-    P[c + st] = P[c];
-    P[c + st + MB_IU * nc] = vel[0]; P[c + st + MB_IV * nc] = vel[1]; P[c + st + MB_IW * nc] = vel[2];
-    P[c + st + MB_IPR * nc] = P[c + MB_IPR * nc];
-    return;
-  }
-  const int nax = dir == 1 ? b.n1 : (dir == 2 ? b.n2 : b.n3);
-  const bool cubic = r.type == 5 || r.type == 6 || (r.type == 11 && nax > 1);
-#pragma unroll
-  for (int s = 0; s < MB_NP; ++s) {
-    double* q0 = P + c + s * nc;
-    const double a1 = q0[0];
-    if (cubic) {  // 3 x1 - 3 x2 + x3, the second layer from the first
-      const double a2 = q0[-st], a3 = q0[-2 * st];
-      const double g1 = 3.0 * a1 - 3.0 * a2 + a3;
-      q0[st] = g1;
-      if (nl > 1) q0[2 * st] = 3.0 * g1 - 3.0 * a1 + a2;
-    } else {
-      q0[st] = a1;
-      if (nl > 1) q0[2 * st] = a1;
-    }
-  }
+  if (q < n) ghost_record(p, rec, list[q], P);
 }
 
 // extrapolation-ghost = cubic on the 400 faces (Fill_Ghost_Cubic_Extrapolation_blk, :859-879),
@@ -198,42 +169,10 @@ __global__ void k_reset_dt(Params p, int only_group) {
     if (only_group < 0 || g == only_group) p.st[g].dtmin_bits = (unsigned long long)__double_as_longlong(1e300);
 }
 
-// the step's dt of every case (Compute_dt's dtglobal = 1e5 then the cell minimum, Mod_Explicit.f90:122;
-// Set_Global_dt; Clip_dt_To_Timemax, Mod_dt.f90:283-296), its simulated time, and a fresh minimum for the
-// next step. A case whose time has reached its stop time (the reference's time-loop exit) is marked done and
-// no longer advances.
 __global__ void k_clock(Params p) {
   pdl_next();
   pdl_wait();
-  for (int g = threadIdx.x; g < p.ngroups; g += blockDim.x) {
-    DevState* st = p.st + g;
-    if (st->done) continue;
-    if (st->t_end > 0.0 && st->time >= st->t_end) {
-      st->done = 1;
-      continue;
-    }
-    // the residual end test of the step just taken (Mod_Explicit.f90:363-370: residuotot(1) <= restop)
-    if (st->res_stop > 0.0 && st->steps > 0 && sqrt(st->res2[0]) <= st->res_stop) {
-      st->done = 1;
-      continue;
-    }
-    // cfl-rise-threshold: the factor of step iter (Mod_dt.f90:57-58); the minimum of the scaled local steps is the
-    // scaled minimum (a product with a positive factor rounds monotonically)
-    const int iter = st->steps + 1;
-    st->rampf = (iter < p.cfl_rise) ? (double)iter / p.cfl_rise : 1.0;
-    double dtg = 1e5;
-    double dm = __longlong_as_double((long long)st->dtmin_bits);
-    dtg = mn(dm * st->rampf, dtg);
-    if (st->time_clip && !p.local_dt) {
-      double rem = st->t_end - st->time;
-      if (rem > 0.0 && dtg > rem) dtg = rem * (1.0 + 1e-12);
-    }
-    st->dt = dtg;
-    if (!p.local_dt) st->time = st->time + dtg;  // time-accurate = false: no simulated time (Mod_Explicit.f90:124-128)
-    st->steps = st->steps + 1;
-    st->dtmin_bits = (unsigned long long)__double_as_longlong(1e300);
-    for (int v = 0; v < MB_NP; ++v) st->res2[v] = 0.0;
-  }
+  clock_groups(p);
 }
 
 // mb_group_reset: case g starts afresh with its stop rule
@@ -251,14 +190,15 @@ __global__ void k_group_reset(Params p, int g, int time_clip, double t_end, doub
 // ---- launchers ----
 static inline unsigned nblk_for(long long n, int t) { return (unsigned)((n + t - 1) / t); }
 
-cudaError_t ghost_fill(const Params& p, const GhostLists& g, double* P, cudaStream_t s, int* nl) {
+cudaError_t ghost_fill(const Params& p, const GhostLists& g, double* P, cudaStream_t s, int* nl, bool clock) {
   *nl = 0;
   if (g.fused) {
     const unsigned nr = nblk_for(g.nphys, 128), ncp = nblk_for(g.ncopy, 128);
-    if (nr + ncp == 0) return cudaSuccess;
+    const unsigned ck = clock ? 1 : 0;
+    if (nr + ncp + ck == 0) return cudaSuccess;
     ++*nl;
-    return launch_chained(p.chain, k_ghost_fill, nr + ncp, 128, 0, s, p, g.rec, g.phys, g.nphys, (int)nr, g.cdst, g.csrc, g.ncopy,
-                          P);
+    return launch_chained(p.chain, k_ghost_fill, nr + ncp + ck, 128, 0, s, p, g.rec, g.phys, g.nphys, (int)nr, g.cdst,
+                          g.csrc, g.ncopy, P, (int)ck);
   }
   if (!g.ordered) {
     if (g.nphys > 0) { k_ghost_phys<<<nblk_for(g.nphys, 128), 128, 0, s>>>(p, g.rec, g.phys, g.nphys, P); ++*nl; }

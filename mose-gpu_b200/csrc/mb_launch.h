@@ -7,11 +7,6 @@
 
 namespace mb {
 
-// a boundary record as the ghost fill needs it
-struct GRec {
-  int blk, i, j, k, face, type;
-};
-
 // the ghost-fill work lists, built by mb_init (device pointers)
 struct GhostLists {
   const GRec* rec;        // every record
@@ -31,6 +26,10 @@ struct GhostLists {
   // fused != 0: no ghost is computed from another ghost of the fill (ordered == 0, and every connection copies interior
   // cells of its donor: the donor is at least two cells deep along its axis), so that one launch fills all of them
   int fused;
+  // surface != 0: fused, and no boundary record reads a ghost (no connections, no viscous symmetry face, and two cells
+  // along the axis where a record reads the cell behind the boundary cell), so that the stage's records, its ghost fill
+  // and the clock share one launch
+  int surface;
   int phys_off[3];
   int cubic_off[3];
 };
@@ -71,7 +70,8 @@ static inline cudaError_t launch_chained(bool chain, void (*kernel)(K...), unsig
   cudaError_t name(const Params& p, const DTile* tiles, int ntiles, int mode, const double* Pin, const double* Pold, \
                    double* Pout, double* Rout, double rkc, int last, int km, cudaStream_t s);                      \
   cudaError_t name##_setup();                                                                                    \
-  cudaError_t name##_records(const Params& p, const RecWork* work, int nrec, const double* P, cudaStream_t s);   \
+  cudaError_t name##_records(const Params& p, const RecWork* work, int nrec, const double* P, const Surface& sf, \
+                             cudaStream_t s);                                                                    \
   cudaError_t name##_dt(const Params& p, const DTile* tiles, int ntiles, const double* P, int only_group,       \
                         cudaStream_t s);                                                                         \
   int name##_occupancy(int visc, int lim);                                                                       \
@@ -99,8 +99,8 @@ MB_DECLARE_SWEEP(sweep_f64f_rs0)
   ((rs) == 1 ? sweep_##form##_rs1##fn args                                                                  \
              : (rs) == 4 ? sweep_##form##_rs4##fn args : (rs) == 12 ? sweep_##form##_rs12##fn args : sweep_##form##_rs0##fn args)
 
-// ghost fill; *nl receives the number of kernels launched
-cudaError_t ghost_fill(const Params& p, const GhostLists& g, double* P, cudaStream_t s, int* nl);
+// ghost fill; *nl receives the number of kernels launched; clock: the fused fill's launch also advances the case clocks
+cudaError_t ghost_fill(const Params& p, const GhostLists& g, double* P, cudaStream_t s, int* nl, bool clock = false);
 cudaError_t dt_cells(const Params& p, const DTile* tiles, int ntiles, const double* P, cudaStream_t s,
                      int only_group = -1);
 cudaError_t update_cells(const Params& p, const DTile* tiles, int ntiles, double* P, const double* PO,
