@@ -859,8 +859,10 @@ int mb_init(const mb_mesh* mesh, const mb_scheme* sc, const mb_thermo* th, int d
   p.n_rk = sc->n_rk; p.irk = 0; p.acc4 = c->d_acc4;
   p.has_pr = sc->prandtl > 0.0;
   p.mach_floor = !(sc->mco >= 1.0);
-  p.cd = {p.ri, p.iri, p.mco, p.has_pr ? 1.0 / p.prandtl : 0.0, (double)p.tmin, (double)(p.tmax - 1)};
-  p.cf = {(float)p.cd.ri, (float)p.cd.iri, (float)p.cd.mco, (float)p.cd.ipr, (float)p.cd.t0, (float)p.cd.t1};
+  p.cd = {p.ri, p.iri, p.mco, p.has_pr ? 1.0 / p.prandtl : 0.0, (double)p.tmin, (double)(p.tmax - 1),
+          p.cfl, 1.0 / p.cfl, p.vnn, 1.0 / p.vnn};
+  p.cf = {(float)p.cd.ri, (float)p.cd.iri, (float)p.cd.mco, (float)p.cd.ipr, (float)p.cd.t0, (float)p.cd.t1,
+          (float)p.cd.cfl, (float)p.cd.icfl, (float)p.cd.vnn, (float)p.cd.ivnn};
   if (cudaMalloc((void**)&c->d_queue, sizeof(int)) != cudaSuccess) { free_ctx(c); return MB_E_NOMEM; }
   {
     int nsm = 0;

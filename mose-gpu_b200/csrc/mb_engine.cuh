@@ -1272,29 +1272,39 @@ MB_HD void prim_update(const Params& p, const double* pc, const double* po, cons
   if (pn[0] < 1e-20) pn[0] = 1e-20;
 }
 
-// The state update of the mixed form: the arithmetic of cons_update, in FP64, with the single-species identities
+// The state update of the simplified path: the arithmetic of cons_update, in FP64, with the single-species identities
 // (rho = rho_s, R_mix = R, h_mix = h(T)) applied exactly and each division by rho, vol or R taken once as a
-// reciprocal: p / rho = R T in the Newton iteration for T, its stop test |de| < 1e-6 |e| without a division. About
-// 30 FP64 divisions fewer per cell; the rounding differs from the parity form's at the last bits.
+// reciprocal: p / rho = R T in the Newton iteration for T, its stop test |de| < 1e-6 |e| without a division; the
+// rounding differs from the parity form's at the last bits. irho, tl: 1 / rho and T of pc, tc: the Newton start (tl
+// inside the thermo guard). A table row and its
+// difference come with one load (Params::tab4). With the local dt below: a step of 192^3 mixed 2.93 and 2.86 ms.
+MB_HD void cp_h_row(const Params& p, double T, double& cp, double& h) {
+  const int ti = tidx(p, T);
+  const double td = T - (double)ti;
+  const double2 a = ldg_(reinterpret_cast<const double2*>(p.tab4) + 2 * ti);
+  const double2 b = ldg_(reinterpret_cast<const double2*>(p.tab4) + 2 * ti + 1);
+  cp = a.x + td * a.y;
+  h = b.x + td * b.y;
+}
 MB_HD void cons_update_fast(const Params& p, const double* pc, const double* po, const double* res, double vol,
-                            double dt, double rkc, double tc, double* pn, long long row_) {
+                            double dt, double rkc, double irho, double tl, double tc, double* pn,
+                            long long row_) {
   const double Rg = p.ri;
   double cons[MB_NP], cold[MB_NP], rl[MB_NP];
-  auto prim2cons = [&](const double* q, double* u) {
-    const double irho = 1.0 / q[0];
+  auto prim2cons = [&](const double* q, double ir, double Tl, double* u) {
     const double vmag = q[MB_IU] * q[MB_IU] + q[MB_IV] * q[MB_IV] + q[MB_IW] * q[MB_IW];
-    const double Tl = q[MB_IPR] * irho * p.iri;
     const int ti = tidx(p, Tl);
-    const double Td = Tl - (double)ti;
-    const double hs = p.h[ti] + Td * (p.h[ti + 1] - p.h[ti]);
-    const double E0 = hs - q[MB_IPR] * irho + 0.5 * vmag;
+    const double2 h = ldg_(reinterpret_cast<const double2*>(p.tab4) + 2 * ti + 1);
+    const double hs = h.x + (Tl - (double)ti) * h.y;
+    const double E0 = hs - q[MB_IPR] * ir + 0.5 * vmag;
     u[0] = q[0];
 #pragma unroll
     for (int s = MB_IU; s <= MB_IW; ++s) u[s] = q[0] * q[s];
     u[MB_IPR] = q[0] * E0;
   };
-  prim2cons(po, cold);
-  prim2cons(pc, cons);
+  prim2cons(pc, irho, tl, cons);
+  const double ir = 1.0 / po[0];
+  prim2cons(po, ir, po[MB_IPR] * ir * p.iri, cold);
   const double f = dt / vol;
 #pragma unroll
   for (int s = 0; s < MB_NP; ++s) rl[s] = -res[s] * f;
@@ -1318,22 +1328,20 @@ MB_HD void cons_update_fast(const Params& p, const double* pc, const double* po,
       for (int s = 0; s < MB_NP; ++s) cons[s] = a4[s * p.nc] + rl[s] * W;
     }
   }
-  const double rho = cons[0], irho = 1.0 / rho;
+  const double rho = cons[0], irn = 1.0 / rho;
   pn[0] = rho;
   double vmag = 0.0;
 #pragma unroll
   for (int s = MB_IU; s <= MB_IW; ++s) {
-    pn[s] = cons[s] * irho;
+    pn[s] = cons[s] * irn;
     vmag = vmag + pn[s] * pn[s];
   }
-  const double energy = cons[MB_IPR] * irho - 0.5 * vmag;
+  const double energy = cons[MB_IPR] * irn - 0.5 * vmag;
   double diff_en = 1e3, T_it = tc;
   int it = 1;
   while ((fabs(diff_en) >= 1e-6 * fabs(energy)) && (it <= 20)) {
-    const int ti = tidx(p, T_it);
-    const double Td = T_it - (double)ti;
-    const double cps = p.cp[ti] + Td * (p.cp[ti + 1] - p.cp[ti]);
-    const double hs = p.h[ti] + Td * (p.h[ti + 1] - p.h[ti]);
+    double cps, hs;
+    cp_h_row(p, T_it, cps, hs);
     const double e_T = hs - Rg * T_it;
     diff_en = fabs(e_T - energy);
     T_it = T_it + (energy - e_T) / (cps - Rg);
@@ -1347,8 +1355,67 @@ MB_HD void cons_update_fast(const Params& p, const double* pc, const double* po,
 // parity form and the standalone Compute_dt, FP32 (geometry and tables in FP32) for the fused dt of the mixed form.
 // PREC: integration-variables = prec, the pseudo-acoustic speed c* = sqrt(alpha^2 u^2 + Ur^2) of the preconditioned
 // system with the cell's Ur (urc) in place of the sound speed (dt_blk.inc:72-75, 89-92, 138-142)
+// On the simplified path: the same rules with |u . m| + a |m| for (|u . m| / |m| + a) |m|, reciprocals for divides and
+// the interleaved tables.
+template <typename R>
+__device__ __forceinline__ R cell_dt_fast(const Params& p, const DBlk& b, long long l, const R* pl) {
+  const R T = pl[MB_IPR] * Cst<R>::of(p).iri * rcp_(pl[0]);
+  R td, cp, h;
+  const int ti = trow<R>(p, T, td);
+  cp_h(p, ti, td, cp, h);
+  const R cv = cp - Cst<R>::of(p).ri;
+  const R a = rsqrt_(cp * Cst<R>::of(p).ri * T * rcp_(cv));
+  R ra_c = (R)0, ra_v = (R)0, dtc = (R)1e8, dv2 = (R)1e30;
+#pragma unroll 1
+  for (int d = 0; d < b.ndir; ++d) {
+    V2<R> xy;
+    R z, dl;
+    metric(b, d, (int)l, xy, z, dl);
+    const R um = fabs(pl[MB_IU] * lo2(xy) + pl[MB_IV] * hi2(xy) + pl[MB_IW] * z);
+    const R g2 = lo2(xy) * lo2(xy) + hi2(xy) * hi2(xy) + z * z;
+    const R gn = rsqrt_(g2);
+    ra_c = ra_c + (um + a * gn);
+    ra_v = ra_v + g2;
+    dtc = mn(dl * Cst<R>::of(p).cfl * rcp_(um * rcp_(gn) + a), dtc);
+    dv2 = mn(dl * dl, dv2);
+  }
+  if (!p.dt_additive) {
+    if (p.visc) {
+      R mu, kap;
+      mu_k(p, T, mu, kap);
+      dtc = mn(pl[0] * Cst<R>::of(p).vnn * rcp_(mu) * dv2, dtc);
+    }
+    return dtc;
+  }
+  if (!p.visc) return Cst<R>::of(p).cfl * rcp_(ra_c);
+  if (b.ndir == 3) {  // the skewness of the cell
+    auto dot = [&](int x, int y) -> R {
+      V2<R> p1, p2;
+      R z1, z2, dd;
+      metric(b, x, (int)l, p1, z1, dd);
+      metric(b, y, (int)l, p2, z2, dd);
+      return lo2(p1) * lo2(p2) + hi2(p1) * hi2(p2) + z1 * z2;
+    };
+    const R g0 = dot(0, 0), g1 = dot(1, 1), g2 = dot(2, 2);
+    const R c12 = dot(0, 1) * rcp_(rsqrt_(g0) * rsqrt_(g1)), c13 = dot(0, 2) * rcp_(rsqrt_(g0) * rsqrt_(g2)),
+            c23 = dot(1, 2) * rcp_(rsqrt_(g1) * rsqrt_(g2));
+    const R ss = c12 * c12 + c13 * c13 + c23 * c23, qp = c12 * c13 * c23;
+    if (ss + (R)2.0 * qp > (R)1.0) {
+      const R mr = (R)2.0 * rsqrt_(ss / (R)3.0) *
+                   cos(acos(mx((R)-1.0, mn((R)1.0, (R)3.0 * rsqrt_((R)3.0) * qp / pow(ss, (R)1.5)))) / (R)3.0);
+      ra_v = ra_v * (R)0.25 * ((R)2.0 + mr + (R)1.0 / mr);
+    }
+  }
+  R mu, kap;
+  mu_k(p, T, mu, kap);
+  const R ir = rcp_(pl[0]);
+  const R Dmx = mx((R)(4.0 / 3.0) * mu * ir, kap * ir * rcp_(cv));
+  return rcp_(ra_c * Cst<R>::of(p).icfl + Dmx * ra_v * Cst<R>::of(p).ivnn);
+}
+
 template <typename R, bool PREC = false>
-MB_HD R cell_dt_t(const Params& p, const DBlk& b, long long l, const R* pl, R urc = (R)0) {
+__device__ __forceinline__ R cell_dt_t(const Params& p, const DBlk& b, long long l, const R* pl, R urc = (R)0) {
+  if constexpr (Fast<R>::on && !PREC) return cell_dt_fast<R>(p, b, l, pl);
   R rho, Rg;
   rotot_rtot(p, pl[0], rho, Rg);
   R Tc = pl[MB_IPR] / (rho * Rg);
@@ -1430,7 +1497,7 @@ MB_HD R cell_dt_t(const Params& p, const DBlk& b, long long l, const R* pl, R ur
   }
   return dtc * (R)1.0;
 }
-MB_HD double cell_dt(const Params& p, const DBlk& b, long long l, const double* pl) {
+__device__ __forceinline__ double cell_dt(const Params& p, const DBlk& b, long long l, const double* pl) {
   return cell_dt_t<double>(p, b, l, pl);
 }
 
@@ -1874,11 +1941,17 @@ __device__ __forceinline__ bool sweep_tile(const Params& p, const DTile t, const
       } else {
         double pc[MB_NP], po[MB_NP], pn[MB_NP];
 #pragma unroll
+        for (int s = 0; s < MB_NP; ++s) pc[s] = ld(Pin + r + s * p.nc);
 #pragma unroll
-        for (int s = 0; s < MB_NP; ++s) { pc[s] = ld(Pin + r + s * p.nc); po[s] = Pold[r + s * p.nc]; }
-        double rho, Tc;
-        if (Fast<R>::on) Tc = pc[MB_IPR] / pc[0] * p.iri;  // one species: R_mix = R
-        else cell_rho_T(p, pc[0], pc[MB_IPR], rho, Tc);
+        for (int s = 0; s < MB_NP; ++s) po[s] = Pold[r + s * p.nc];
+        double rho, Tc, irho = 0.0;
+        if (Fast<R>::on) {  // one species: R_mix = R
+          irho = 1.0 / pc[0];
+          Tc = pc[MB_IPR] * irho * p.iri;
+        } else {
+          cell_rho_T(p, pc[0], pc[MB_IPR], rho, Tc);
+        }
+        const double Tl = Tc;
         if (p.guard && !(Tc > 1.0 && Tc < 9990.0)) {  // thermo guard (Mod_Thermo_Cache.f90:317-327)
           atomicAdd(&st->n_bad_thermo, 1);
           if (Tc != Tc) Tc = 300.0;
@@ -1895,7 +1968,7 @@ __device__ __forceinline__ bool sweep_tile(const Params& p, const DTile t, const
           dtc = (double)cell_dt_t<R>(p, b, r - b.boff, pr) * st->rampf;
         }
         if (RS == 0 && p.intvar) prim_update(p, pc, po, acc, vol, dtc, rkc, pn, p.prec ? ld(p.ur + r) : 0.0);
-        else if (Fast<R>::on) cons_update_fast(p, pc, po, acc, vol, dtc, rkc, Tc, pn, r);
+        else if (Fast<R>::on) cons_update_fast(p, pc, po, acc, vol, dtc, rkc, irho, Tl, Tc, pn, r);
         else cons_update(p, pc, po, acc, vol, dtc, rkc, Tc, pn, r);
         bool bad = !(pn[MB_IPR] >= 0.0);
 #pragma unroll

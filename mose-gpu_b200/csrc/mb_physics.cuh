@@ -122,6 +122,7 @@ struct FluxCst {
   R ri, iri;   // gas constant and its reciprocal
   R mco, ipr;  // Mco, 1 / Prandtl (0 without one)
   R t0, t1;    // first and last table row that starts an interval
+  R cfl, icfl, vnn, ivnn;
 };
 
 struct Params {
