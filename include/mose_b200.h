@@ -462,7 +462,7 @@ int mb_get_tuning(const mb_ctx* ctx, int* kchunk, int* persistent, float* ms);
 /* The tile staging of the mixed form's sweep (no counterpart in the reference): tma = 1 (the default) stages each
  * plane of a tile by TMA, cp.async.bulk.tensor boxes of 38 rows x 5 variables of the state arena landing on an
  * mbarrier (bounded waits; a wait that gives up sets MB_E_TIMEOUT in the case status), converted into a 5-value
- * FP32 tile (rho, u, v, w, T; p = rho R T where it is read) with the k-face fluxes carried in registers; tma = 0
+ * FP32 tile (rho, u, v, w, T; p = rho R T where it is read); tma = 0
  * stages by per-thread coalesced loads into a 6-value tile (rho, u, v, w, p, T). The two differ in the FP32
  * rounding of p (within the mixed form's accuracy); mb_autotune keeps the faster for each tile list (this call sets
  * both lists: the blocks with several k planes, and the mirrored one-plane blocks). TMA is used where a tensor map of

@@ -1,7 +1,8 @@
 // mb_engine.cuh -- kernels of the B200 engine.
 //
 //   k_sweep      the fused stage: every interior face flux of a tile computed ONCE (one thread per
-//                face), exchanged through shared memory, summed per cell in the reference's pass-2
+//                face), exchanged through shared memory (the simplified path: partly in registers
+//                and by shuffles), summed per cell, in the FP64 parity form in the reference's pass-2
 //                order (src/lib/gpu/pass2_body.inc), the boundary records of the cell added in face
 //                order 1..6 (numerics/fluxes/bc/Mod_BC.f90:449-485), then either the residual is
 //                written (parity hook, mode RESIDUAL) or the conservative RK update is applied
@@ -14,8 +15,8 @@
 // Tiling: a CTA owns a tile of 32 (i) x TY (j) cells of one block and marches over a chunk of k
 // planes. Per plane it computes the (32+1) x TY i-faces, 32 x (TY+1) j-faces and the 32 x TY
 // k-faces above the plane (the k-face below is the previous plane's), so only the tile's left i-faces
-// and bottom j-faces are computed twice across CTAs. Warps run the face tasks through one call
-// site, which keeps a single copy of the flux code in the kernel.
+// and bottom j-faces are computed twice across CTAs. The statement-order form runs its long face code
+// through one call site for all directions; the simplified path (PAIR) has one per direction.
 #pragma once
 #include "mb_pair.cuh"
 #include "mb_physics.cuh"
@@ -48,15 +49,15 @@ template <typename R> MB_HD R cvt(double x) { return (R)x; }
 // that one shared load brings two values; each kind holds all its slots, so a cell has one offset for all of them.
 constexpr int TXH = 36;
 // The staging of a sweep's state tile, a template parameter of the sweep (STG) chosen per context (mb_autotune,
-// mb_set_staging): STG_PLAIN, per-thread coalesced loads into a 6-value tile (rho_s, u, v, w, p, T) with the k-face
-// fluxes of two planes in shared memory; STG_TMA (the mixed form), TMA boxes of the state arena landing on an mbarrier
-// in a staging buffer, converted into a 5-value tile (rho_s, u, v, w, T; p = rho Rg T where it is read) with the
-// k-face fluxes carried in registers, which together leave room for the staging buffer at 3 CTAs per SM.
+// mb_set_staging): STG_PLAIN, per-thread coalesced loads into a 6-value tile (rho_s, u, v, w, p, T); STG_TMA (the
+// mixed form), TMA boxes of the state arena landing on an mbarrier in a staging buffer, converted into a 5-value tile
+// (rho_s, u, v, w, T; p = rho Rg T where it is read), which leaves room for the staging buffer at 3 CTAs per SM (the
+// run-time solver unit, which exchanges every face through shared memory, also keeps its k-face fluxes in registers).
 enum { STG_PLAIN = 0, STG_TMA = 1 };
 template <typename R, int STG> struct Stg {
   static constexpr bool tma = STG == STG_TMA && sizeof(R) == 4;
   static constexpr int nv = tma ? 5 : 6;   // values per staged cell
-  static constexpr bool kreg = tma;        // k-face fluxes in registers
+  static constexpr bool kreg = tma;        // k-face fluxes in registers (run-time solver unit)
 };
 
 // the plane slot of plane kk (kk >= -1); the tile of a mirrored one-plane block (KM) holds its one plane only
@@ -1703,19 +1704,29 @@ __device__ __forceinline__ bool sweep_tile(const Params& p, const DTile t, const
   T.base = reinterpret_cast<R*>(smem_raw);                                       // the state tile
   T.rg = (R)p.ri;
   unsigned char* fbase = smem_raw + sizeof(R) * tile_planes<KM>() * NVT * (TY + 4) * TXH;
+  // the simplified flux path (PAIR): a thread sums the net fluxes of its cell's faces as it computes them (its left and
+  // lower faces; the right one comes from the next lane by a shuffle, the k-face below from a slot of its own) and only
+  // the j-faces, and the i-faces right of the tile, go through shared memory: 52 KB a CTA instead of 63, which leaves the
+  // L1 92 KB instead of 60, and 20 shared accesses a cell fewer. One B200, a step with all faces exchanged and so: 192^3
+  // mixed 2.86 and 2.82 ms, duct 348 and 320 us, eight steps of 2-D 301^2 542 and 515 us, 96^3 FP64 production 1.35 and
+  // 1.27 ms.
+  // The two fluxes of an axis are subtracted before anything is added to their difference, which in FP32 loses nothing of
+  // the pressure they share.
+  RowJ* sJ = reinterpret_cast<RowJ*>(fbase);                                      // [TY+1][32][NS] face below row r
+  RowJ* sK = sJ + TY + 1;                                                         // [TY][32][NS] the k-face below
+  R* sX = reinterpret_cast<R*>(KM ? sK : sK + TY);                                // [2][TY][NS] left and right face of a
+                                                                                  // row's last cell
   RowI* sFi = reinterpret_cast<RowI*>(fbase);                                     // [TY][33][NS]
   RowJ* sFj = reinterpret_cast<RowJ*>(fbase + sizeof(R) * TY * 33 * NS);          // [TY+1][32][NS]
   // the k-faces: the face above a cell is computed by the thread of that cell and is the face below it on the next
-  // plane, so the mixed form carries both in that thread's registers (kup, kdn: no shared buffer, which leaves room
-  // for the TMA staging buffer at 3 CTAs per SM); the FP64 forms keep them in shared memory (two planes)
-  constexpr bool KREG = Stg<R, STG>::kreg;
-  RowJ* sFk0 = reinterpret_cast<RowJ*>(fbase + sizeof(R) * (TY * 33 + (TY + 1) * 32) * NS);  // [2][TY][32][NS]
+  // plane: it stays in that thread's registers until pass 2 (kup) and then goes to a slot of its own in shared memory,
+  // or, with TMA staging (KREG), stays in registers (kdn) to leave room for the staging buffer. One plane of slots, not
+  // two, lets the FP64 parity form hold tiles of 5 rows at 2 CTAs per SM.
+  constexpr bool KREG = Stg<R, STG>::kreg && !PAIR;
+  RowJ* sFk0 = reinterpret_cast<RowJ*>(fbase + sizeof(R) * (TY * 33 + (TY + 1) * 32) * NS);  // [TY][32][NS]
   R kup[NS], kdn[NS];
 #pragma unroll
   for (int q = 0; q < NS; ++q) kup[q] = kdn[q] = (R)0;
-  // the block in shared memory: a local copy went to the stack (its record maps are indexed at run time), and its fields
-  // came back through local loads. A step with the stack copy and so: 2-D batch 693 and 588 us, 16 served cases 3.04 and
-  // 2.59 ms, 192^3 mixed 3.11 and 3.07 ms.
   for (int w = threadIdx.x; w < (int)(sizeof(DBlk) / 4); w += blockDim.x)
     reinterpret_cast<int*>(&sblk)[w] = __ldg(reinterpret_cast<const int*>(p.blk + t.blk) + w);
   __syncthreads();
@@ -1731,7 +1742,6 @@ __device__ __forceinline__ bool sweep_tile(const Params& p, const DTile t, const
   const double dt = (MODE == MODE_UPDATE) ? st->dt : 0.0;
   double dtloc = 1e300;
   if (MODE == MODE_UPDATE && last && tid < 8 * MB_NP) s_res[tid] = 0.0;  // used after the prologue's barrier
-  int kb = 0;  // buffer of the k-face above the current plane
   // ghost layers the stencils read: 2 along an axis with faces; for a block one cell deep along j or k (2-D,
   // 1-D) no face of that axis exists and only the viscous transverse gradient reads one ghost layer
   const bool sens = RS == 0 && p.sd;  // the shock sensor reads the six face neighbours of a cell
@@ -1768,7 +1778,7 @@ __device__ __forceinline__ bool sweep_tile(const Params& p, const DTile t, const
 #pragma unroll
       for (int q = 0; q < NS; ++q) kdn[q] = NET ? out[q] - out[MB_NP + q] : out[q];
     } else {
-      R* dst = &sFk0[(kb ^ 1) * TY + ty][tx][0];
+      R* dst = PAIR ? &sK[ty][tx][0] : &sFk0[ty][tx][0];
 #pragma unroll
       for (int q = 0; q < NS; ++q) dst[q] = NET ? out[q] - out[MB_NP + q] : out[q];
     }
@@ -1794,42 +1804,57 @@ __device__ __forceinline__ bool sweep_tile(const Params& p, const DTile t, const
     if (tma && k + 3 <= b.n3 + kext && k + 1 < t.k1) tma_issue_plane<TY>(p, b, raw, bar, t.i0, t.j0, k + 3);
     // ---- face tasks of this plane through one call site: 0 = i-face #tid, 1 = extra i-faces (last warp,
     // lanes < TY), 2 = j-face #tid, 3 = extra j-face row (warp 0), 4 = the k-face above
+    R net[NS];
     if constexpr (PAIR) {
       // one call site per direction: with a literal d the offsets and pointers need no selects, and the shorter face code
-      // no longer crowds the instruction cache. One B200, a step with one call site for all and so: 192^3 mixed 3.06 and
-      // 2.95 ms, the 12-block 2-D batch 577 and 527 us, eight steps of 2-D 301^2 707 and 662 us.
+      // no longer crowds the instruction cache (one B200, a step with one call site for all and so: 192^3 mixed 3.06 and
+      // 2.95 ms, the 12-block 2-D batch 577 and 527 us). The tile's extra faces come first, before a thread holds sums.
 #pragma unroll 1
-      for (int rep = 0; rep < 2; ++rep) {  // i-faces
-        if (rep == 1 && (ty != TY - 1 || tx >= TY)) break;
-        const int f = rep == 0 ? tid : 32 * TY + tx;
-        const int rw = f / 33, cl = f - rw * 33;
-        const int fi = t.i0 + cl - 1, fj = t.j0 + rw;
-        if (fi >= 1 && fi <= b.n1 - 1 && fj <= b.n2) {
+      for (int rep = 0; rep < 2; ++rep) {  // j: warp 0 the faces above the tile's last row; every cell's lower face
+        if (rep == 0 && ty != 0) continue;
+        const int rw = rep == 0 ? TY : ty, fj = t.j0 + rw - 1;
+        if (fj >= 1 && fj <= b.n2 - 1 && i <= b.n1) {
           R out[NF];
-          face_fast<R, TY, VISC, RS, LIM, KM, NVT>(p, b, T, 0, fi, fj, k, cl + 1, rw + 2, out);
+          face_fast<R, TY, VISC, RS, LIM, KM, NVT>(p, b, T, 1, i, fj, k, tx + 2, rw + 1, out);
 #pragma unroll
-          for (int q = 0; q < NS; ++q) sFi[rw][cl][q] = out[q];
+          for (int q = 0; q < NS; ++q) sJ[rw][tx][q] = out[q];
         }
       }
 #pragma unroll 1
-      for (int rep = 0; rep < 2; ++rep) {  // j-faces
-        if (rep == 1 && ty != 0) break;
-        const int rw = rep == 0 ? ty : TY;
-        const int fi = t.i0 + tx, fj = t.j0 + rw - 1;
-        if (fj >= 1 && fj <= b.n2 - 1 && fi <= b.n1) {
-          R out[NF];
-          face_fast<R, TY, VISC, RS, LIM, KM, NVT>(p, b, T, 1, fi, fj, k, tx + 2, rw + 1, out);
-#pragma unroll
-          for (int q = 0; q < NS; ++q) sFj[rw][tx][q] = out[q];
-        }
-      }
-      if (!KM && own && k < b.n3) {  // the k-face above
+      for (int rep = 0; rep < 2; ++rep) {  // i: the last warp the faces right of the tile; every cell's left face
+        if (rep == 0 && (ty != TY - 1 || tx >= TY)) continue;
+        const int fi = rep == 0 ? t.i0 + 31 : i - 1, fj = rep == 0 ? t.j0 + tx : j;
         R out[NF];
-        face_fast<R, TY, VISC, RS, LIM, KM, NVT>(p, b, T, 2, i, j, k, tx + 2, ty + 2, out);
+#pragma unroll
+        for (int q = 0; q < NS; ++q) out[q] = (R)0;
+        if (fi >= 1 && fi <= b.n1 - 1 && fj <= b.n2)
+          face_fast<R, TY, VISC, RS, LIM, KM, NVT>(p, b, T, 0, fi, fj, k, fi - t.i0 + 2, fj - t.j0 + 2, out);
+        if (rep == 0) {
+#pragma unroll
+          for (int q = 0; q < NS; ++q) sX[(TY + tx) * NS + q] = out[q];
+        } else {
+          __syncwarp();
+#pragma unroll
+          for (int q = 0; q < NS; ++q) {
+            const R up = __shfl_down_sync(0xffffffffu, out[q], 1);
+            net[q] = tx < 31 ? up - out[q] : (R)0;
+          }
+          if (tx == 31) {  // its right face is another warp's: pass 2 takes the difference
+#pragma unroll
+            for (int q = 0; q < NS; ++q) sX[ty * NS + q] = out[q];
+          }
+        }
+      }
+      if (!KM && own) {  // the k-face above, and the one below (the last plane's)
+        R* kf = &sK[ty][tx][0];
+        R out[NF];
+#pragma unroll
+        for (int q = 0; q < NS; ++q) out[q] = (R)0;
+        if (k < b.n3) face_fast<R, TY, VISC, RS, LIM, KM, NVT>(p, b, T, 2, i, j, k, tx + 2, ty + 2, out);
 #pragma unroll
         for (int q = 0; q < NS; ++q) {
-          if (KREG) kup[q] = out[q];
-          else sFk0[kb * TY + ty][tx][q] = out[q];
+          net[q] = net[q] + (out[q] - (k > 1 ? kf[q] : (R)0));
+          kf[q] = out[q];
         }
       }
     } else {
@@ -1853,13 +1878,12 @@ __device__ __forceinline__ bool sweep_tile(const Params& p, const DTile t, const
         if (fj >= 1 && fj <= b.n2 - 1 && fi <= b.n1) { d = 1; dst = &sFj[rw][cl][0]; }
       } else {
         if (!own || k >= b.n3) continue;
-        fi = i; fj = j; ii = tx + 2; jj = ty + 2; d = 2; dst = KREG ? nullptr : &sFk0[kb * TY + ty][tx][0];
+        fi = i; fj = j; ii = tx + 2; jj = ty + 2; d = 2;
       }
       if (d < 0) continue;
       R out[NF];
-      if constexpr (PAIR) face_fast<R, TY, VISC, RS, LIM, KM, NVT>(p, b, T, d, fi, fj, k, ii, jj, out);
-      else face_flux<R, TY, VISC, RS, LIM, KM, NVT>(p, b, T, d, fi, fj, k, ii, jj, out);
-      if (KREG && task == 4) {
+      face_flux<R, TY, VISC, RS, LIM, KM, NVT>(p, b, T, d, fi, fj, k, ii, jj, out);
+      if (task == 4) {
 #pragma unroll
         for (int q = 0; q < NS; ++q) kup[q] = NET ? out[q] - out[MB_NP + q] : out[q];
       } else {
@@ -1882,31 +1906,34 @@ __device__ __forceinline__ bool sweep_tile(const Params& p, const DTile t, const
       const R* gr = (j < b.n2) ? &sFj[ty + 1][tx][0] : nullptr;
       const R* gl = (j > 1) ? &sFj[ty][tx][0] : nullptr;
       const bool hr_on = k < b.n3, hl_on = k > 1;
-      const R* hr = (!KREG && hr_on) ? &sFk0[kb * TY + ty][tx][0] : nullptr;
-      const R* hl = (!KREG && hl_on) ? &sFk0[(kb ^ 1) * TY + ty][tx][0] : nullptr;
+      const R* hl = &sFk0[ty][tx][0];
       // the sum runs in the flux type (the FP64 form: FP64 in the reference's order; the mixed form: the six FP32
       // net face fluxes summed in FP32 and converted once), the boundary records and the update in FP64
 #pragma unroll
       for (int s = 0; s < MB_NP; ++s) {
         R a = (R)0;
+        if constexpr (PAIR) {
+          R g = (R)0;
+          if (j < b.n2) g = sJ[ty + 1][tx][s];
+          if (j > 1) g = g - sJ[ty][tx][s];
+          a = net[s] + g;
+          if (tx == 31) a = a + ((i < b.n1 ? sX[(TY + ty) * NS + s] : (R)0) - sX[ty * NS + s]);
+          acc[s] = (double)a;
+          continue;
+        }
         if (fr) a = a + fr[s];
         if (fl) a = a - fl[s];
         if (gr) a = a + gr[s];
         if (gl) a = a - gl[s];
-        if (KREG) {
-          if (hr_on) a = a + kup[s];
-          if (hl_on) a = a - kdn[s];
-        } else {
-          if (hr) a = a + hr[s];
-          if (hl) a = a - hl[s];
-        }
+        if (hr_on) a = a + kup[s];
+        if (hl_on) a = a - (KREG ? kdn[s] : hl[s]);
         if (VISC && !NET && !PAIR) {
           if (fr) a = a - fr[MB_NP + s];
           if (fl) a = a + fl[MB_NP + s];
           if (gr) a = a - gr[MB_NP + s];
           if (gl) a = a + gl[MB_NP + s];
-          if (hr) a = a - hr[MB_NP + s];
-          if (hl) a = a + hl[MB_NP + s];
+          if (hr_on) a = a - kup[MB_NP + s];
+          if (hl_on) a = a + hl[MB_NP + s];
         }
         acc[s] = (double)a;
       }
@@ -1974,8 +2001,6 @@ __device__ __forceinline__ bool sweep_tile(const Params& p, const DTile t, const
 #pragma unroll
         for (int s = 0; s < MB_NP; ++s) bad = bad || !isfinite(pn[s]);
         if (bad) report_bad_state(st, t.blk, i, j, k);
-#pragma unroll
-        for (int s = 0; s < MB_NP; ++s) Pout[r + s * p.nc] = pn[s];
         if (last) {  // the new state's local dt, in the flux type (FP64 in the parity form)
 #pragma unroll
           for (int v = 0; v < MB_NP; ++v) {
@@ -1987,6 +2012,8 @@ __device__ __forceinline__ bool sweep_tile(const Params& p, const DTile t, const
           for (int s = 0; s < MB_NP; ++s) pr[s] = cvt<R>(pn[s]);
           dtloc = mn(dtloc, (double)cell_dt_t<R>(p, b, r - b.boff, pr));
         }
+#pragma unroll
+        for (int s = 0; s < MB_NP; ++s) Pout[r + s * p.nc] = pn[s];
       }
     }
     if (MODE == MODE_UPDATE && last) {  // uniform over the CTA: each warp adds its plane sums into its own slots
@@ -1998,10 +2025,12 @@ __device__ __forceinline__ bool sweep_tile(const Params& p, const DTile t, const
         if ((tid & 31) == 0) s_res[8 * v + (tid >> 5)] += (double)x;
       }
     }
-    kb ^= 1;
-    if (KREG) {
+    if (!PAIR && own && k < b.n3) {
 #pragma unroll
-      for (int q = 0; q < NS; ++q) kdn[q] = kup[q];
+      for (int q = 0; q < NS; ++q) {
+        if (KREG) kdn[q] = kup[q];
+        else if (!KM) sFk0[ty][tx][q] = kup[q];
+      }
     }
   }
   if (MODE == MODE_UPDATE && last) {
@@ -2018,15 +2047,18 @@ __device__ __forceinline__ bool sweep_tile(const Params& p, const DTile t, const
 // shared memory of the sweep: the state tile and the face-flux buffers (sweep_smem_core), and in the mixed form the
 // TMA staging buffer of one plane (TY+4 row slots) with its 128-byte alignment slack. The tiles of mirrored one-plane
 // blocks (KM) hold one plane and have no k faces (no k-face buffers): a quarter of the tile, more CTAs per SM
-template <typename R, int TY, bool VISC, int STG = STG_PLAIN, bool KM = false>
+template <typename R, int TY, bool VISC, int STG = STG_PLAIN, bool KM = false, bool PAIR = false>
 MB_HD constexpr size_t sweep_smem_core() {
+  if (PAIR)  // j-faces, k-faces below, i-faces right of the tile
+    return sizeof(R) * ((size_t)tile_planes<KM>() * Stg<R, STG>::nv * (TY + 4) * TXH +
+                        (size_t)((KM ? 1 : 2) * TY * 32 + 32 + 2 * TY) * MB_NP);
   return sizeof(R) * ((size_t)tile_planes<KM>() * Stg<R, STG>::nv * (TY + 4) * TXH +
-                      (size_t)(TY * 33 + (TY + 1) * 32 + ((Stg<R, STG>::kreg || KM) ? 0 : 2 * TY * 32)) *
+                      (size_t)(TY * 33 + (TY + 1) * 32 + ((Stg<R, STG>::kreg || KM) ? 0 : TY * 32)) *
                           ((VISC && !Fast<R>::on) ? 2 * MB_NP : MB_NP));
 }
-template <typename R, int TY, bool VISC, int STG = STG_PLAIN, bool KM = false>
+template <typename R, int TY, bool VISC, int STG = STG_PLAIN, bool KM = false, bool PAIR = false>
 MB_HD constexpr size_t sweep_smem() {
-  return sweep_smem_core<R, TY, VISC, STG, KM>() +
+  return sweep_smem_core<R, TY, VISC, STG, KM, PAIR>() +
          (Stg<R, STG>::tma ? (size_t)128 + (size_t)(TY + 4) * TMA_ROW_BYTES : 0);
 }
 
@@ -2051,7 +2083,7 @@ k_sweep(Params p, const DTile* __restrict__ tiles, const double* __restrict__ Pi
   pdl_next();
   TmaStage ts{nullptr, &s_bar, 0u};
   if (Stg<R, STG>::tma) {  // the staging buffer after the tile and the flux buffers, 128-byte aligned
-    unsigned char* q = smem_raw + sweep_smem_core<R, TY, VISC, STG, KM>();
+    unsigned char* q = smem_raw + sweep_smem_core<R, TY, VISC, STG, KM, Fast<R>::on && RS != 0>();
     ts.halo = q + ((128u - (smem_addr(q) & 127u)) & 127u);
     if (p.tmap) {
       if (threadIdx.x == 0) mbar_init(&s_bar);
