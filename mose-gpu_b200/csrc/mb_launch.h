@@ -34,10 +34,11 @@ struct GhostLists {
   int cubic_off[3];
 };
 
-constexpr int TY_F64 = 4;    // tile rows of the FP64 parity sweep (128 threads)
-constexpr int TY_F64F = 6;   // tile rows of the FP64 production sweep: 192 threads at 168 registers, 12 warps per SM and
-                             // fewer j-faces computed twice than 4 rows (128 threads, 232 registers, 8 warps per SM):
-                             // a step of 96^3 1.71 and 1.45 ms, of the 4-block 2-D batch 370 and 312 us
+constexpr int TY_F64 = 5;    // tile rows of the FP64 parity sweep: 160 threads at 168 registers, 10 warps per SM; 4 rows
+                             // (232 registers, 8 warps) took 1.37 ms for a step of 64^3, these 1.07 ms; 160^3 the same
+constexpr int TY_F64F = 8;   // tile rows of the FP64 production sweep: 256 threads at 128 registers, 16 warps per SM and an
+                             // eighth of the j-faces computed twice. A step of 96^3: 4 rows (128 threads, 232 registers,
+                             // 8 warps per SM) 1.71 ms, 6 rows (168 registers, 12 warps) 1.27 ms, 8 rows 1.14 ms
 constexpr int TY_F32 = 8;    // tile rows of the mixed sweep (256 threads)
 constexpr int MINB_F64 = 2;  // resident CTAs per SM the FP64 sweep's registers must allow
 constexpr int MINB_F32 = 3;  // resident CTAs per SM the mixed sweep's registers must allow (80 registers)
