@@ -69,6 +69,7 @@ struct mb_ctx {
   bool no_tma = false;          // MB_NO_TMA set at mb_init: no tensor maps (the TMA staging is never used)
   bool stage_tma = true;        // the mixed sweep stages by TMA where a map exists (mb_set_staging, mb_autotune)
   bool stage_tma_km = true;     // the same for the tile list of mirrored one-plane blocks (tuned separately)
+  bool dense = false;           // Params::dense of the main tile list (mb_autotune, with plain staging)
   cudaStream_t tstream = 0;     // the stream the mesh tables are (re)built in the order of (build_tables)
   long long sweeps_tma = 0, sweeps_plain = 0;  // sweep launches of the mixed form by staging path
   double* d_acc4 = nullptr;     // RK4: conserved accumulator (ncell x 5)
@@ -240,7 +241,8 @@ int mb_selftest_bounded_wait(int device, int tries, int* gave_up) {
 
 int mb_set_staging(mb_ctx* ctx, int tma) {
   if (!ctx || tma < 0 || tma > 1) return MB_E_ARG;
-  if (ctx->stage_tma != (tma == 1) || ctx->stage_tma_km != (tma == 1)) {
+  if (ctx->stage_tma != (tma == 1) || ctx->stage_tma_km != (tma == 1) || ctx->dense) {
+    ctx->dense = false;
     ctx->stage_tma = tma == 1;
     ctx->stage_tma_km = tma == 1;
     if (ctx->gexec) { cudaGraphExecDestroy(ctx->gexec); ctx->gexec = nullptr; }  // a replay in flight completes
@@ -873,6 +875,7 @@ int mb_init(const mb_mesh* mesh, const mb_scheme* sc, const mb_thermo* th, int d
     p.pgrid = std::max(1, occ) * std::max(1, nsm);
     int occ_km = MB_BY_FORM(sc->precision, sweep_unit(sc), _occupancy_km, (v, sc->limiter));
     p.pgrid_km = std::max(1, occ_km) * std::max(1, nsm);
+    p.pgrid_dense = MB_BY_FORM(sc->precision, sweep_unit(sc), _occupancy_dense, (v, sc->limiter)) * std::max(1, nsm);
   }
   p.queue = nullptr;
   // ---- the mesh tables
@@ -1048,6 +1051,7 @@ static int sweep_on(mb_ctx* c, const DTile* t, int n, int persistent, int mode, 
   p.irk = irk;
   p.queue = persistent ? c->d_queue : nullptr;
   p.stg = (c->sc.precision == MB_PREC_MIXED && (km ? c->stage_tma_km : c->stage_tma)) ? STG_TMA : STG_PLAIN;
+  p.dense = c->dense && !km;
   p.tmap = p.stg == STG_TMA ? tmap_of(c, Pin, s, false) : nullptr;
   if (c->sc.precision == MB_PREC_MIXED) (p.tmap ? c->sweeps_tma : c->sweeps_plain) += 1;
   const double rkc = irk > 0 ? rkc_of(c->sc.n_rk, irk) : 0.0;
@@ -1569,7 +1573,8 @@ int mb_get_status(mb_ctx* ctx, mb_status* st) { return mb_get_group_status(ctx, 
 //  - for the main tile list and, separately, for the tiles of the mirrored one-plane blocks (2-D meshes): a plain
 //    grid of one CTA per tile against the persistent work queue (about one wave of CTAs taking tiles, largest first,
 //    from a counter);
-//  - the mixed form: the tile staging (TMA boxes into a 5-value tile, or plain loads into a 6-value tile).
+//  - the mixed form: the tile staging (TMA boxes into a 5-value tile, or plain loads into a 6-value tile), and of the
+//    3-D tiles the plain staging at 4 CTAs per SM.
 // The k-chunk and the queue never change a result; the staging changes the FP32 rounding of p in the mixed form.
 int mb_autotune(mb_ctx* ctx, const double* P, void* stream) {
   if (!ctx || !P) return MB_E_ARG;
@@ -1577,6 +1582,7 @@ int mb_autotune(mb_ctx* ctx, const double* P, void* stream) {
   cudaStream_t s = (cudaStream_t)stream;
   prepare_tmaps(ctx, P, P, s);
   const int ty = ctx->ty_sweep;
+  ctx->dense = false;
   int rc;
   long long ccells[4] = {0, 0, 0, 0};
   int cmaxk[4] = {0, 0, 0, 0};
@@ -1645,7 +1651,22 @@ int mb_autotune(mb_ctx* ctx, const double* P, void* stream) {
     }
     ctx->stage_tma = ms_stage[1] < ms_stage[0];
     ctx->stage_tma_km = ms_stage_km[1] < ms_stage_km[0];
-    ctx->tuned_ms = std::min(ms_stage[0], ms_stage[1]) + std::min(ms_stage_km[0], ms_stage_km[1]);
+    float best = std::min(ms_stage[0], ms_stage[1]);
+    // the 3-D sweep at 4 CTAs per SM instead of 3: a third more warps to cover latency, but 64 registers and an L1 of
+    // 28 KB instead of 92. It wins where the geometry stays in the caches (one B200, 64 blocks of 32^3 that share it, a
+    // step 1215 and 1068 us) and loses where it streams (192^3 in one block 2.82 and 3.03 ms), so it is timed
+    if (!use.empty() && ctx->p.pgrid_dense > ctx->p.pgrid) {
+      const bool tma = ctx->stage_tma;
+      float ms = 0.f;
+      ctx->stage_tma = false;
+      ctx->dense = true;
+      rc = time_sweep(ctx, use, ctx->persistent, P, 3, s, &ms);
+      ctx->dense = rc == MB_OK && ms < best;
+      if (!ctx->dense) ctx->stage_tma = tma;
+      if (rc != MB_OK) return rc;
+      best = std::min(best, ms);
+    }
+    ctx->tuned_ms = best + std::min(ms_stage_km[0], ms_stage_km[1]);
   }
   for (auto* d : {&ctx->d_tiles_sweep, &ctx->d_tiles_km}) {
     if (*d) cudaFree(*d);
@@ -1684,6 +1705,7 @@ int mb_set_tuning(mb_ctx* ctx, int kchunk, int persistent) {
   CK(cudaDeviceSynchronize());
   ctx->kc3 = kchunk;
   ctx->tuned = true;
+  ctx->dense = false;
   for (int c = 0; c < 4; ++c) ctx->kcls[c] = kchunk;
   ctx->persistent = persistent;
   std::vector<DTile> use = make_tiles(ctx->hdims, ctx->ty_sweep, kchunk, 0xe, &ctx->hkm, 0);

@@ -76,6 +76,7 @@ static inline cudaError_t launch_chained(bool chain, void (*kernel)(K...), unsig
   cudaError_t name##_dt(const Params& p, const DTile* tiles, int ntiles, const double* P, int only_group,       \
                         cudaStream_t s);                                                                         \
   int name##_occupancy(int visc, int lim);                                                                       \
+  int name##_occupancy_dense(int visc, int lim);                                                                 \
   int name##_occupancy_km(int visc, int lim);
 MB_DECLARE_SWEEP(sweep_f64_rs1)
 MB_DECLARE_SWEEP(sweep_f64_rs4)

@@ -163,6 +163,8 @@ struct Params {
   int* queue;              // persistent sweep: the tile counter (null: one CTA per tile)
   int ntiles_run;          // tiles of the launch (persistent sweep)
   int chain;               // the launches of a stage are chained (launch_chained): the mesh has at most one tile per SM
+  int dense;               // 3-D mixed sweep at 4 CTAs per SM (64 registers) instead of 3 (80); its persistent grid
+  int pgrid_dense;
   int pgrid;               // CTAs of a persistent launch (resident CTAs per SM x SMs)
   int pgrid_km;            // the same for the tiles of mirrored one-plane blocks (their own occupancy)
   int n_rk;                // 4: classical RK4 through the accumulator acc4
