@@ -13,6 +13,7 @@ Units compile in parallel. Usage: python mose-gpu_b200/build.py [--force] [-v]
 import os
 import subprocess
 import sys
+import time
 from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
@@ -51,7 +52,10 @@ def build(force=False, verbose=False):
 
     def run(job):
         src, cmd = job
+        began = time.time()
         r = subprocess.run(cmd, capture_output=True, text=True)
+        if r.returncode == 0:  # the object is as old as what it was compiled from: a header edited meanwhile rebuilds it
+            os.utime(cmd[-1], (began, began))
         return src, r
 
     logs = []
@@ -61,7 +65,7 @@ def build(force=False, verbose=False):
             if r.returncode != 0:
                 sys.stderr.write(r.stderr)
                 raise RuntimeError("nvcc failed on %s" % src)
-    if force or _mtime(OUT) < max(_mtime(o) for o in objs):
+    if force or jobs or _mtime(OUT) < max(_mtime(o) for o in objs):
         cmd = [NVCC] + ARCH + ["-shared", "-cudart", "static", "-o", OUT] + objs
         r = subprocess.run(cmd, capture_output=True, text=True)
         if r.returncode != 0:
