@@ -1,0 +1,119 @@
+"""The simplified flux path (paired values, faces summed in registers, shuffles and shared exchange rows) and the merged
+surface launches at the sizes where they can go wrong: one cell below, at and above the 32 x 8 tiles, axes of one to three
+cells, every limiter, the three solvers with their own unit, walls, inlet, outflow, symmetry and connections.
+
+Tolerances: the FP64 production form against the oracle at the north-star gate of one step (1e-12, max-norm relative to
+the field, momentum against its vector); the parity form bit for bit. The mixed form: every face flux carries a few FP32
+roundings of the state's own size (p and rho u H), so a step moves the conserved variables by at most about
+3 faces x 8 roundings x 2^-24 x the CFL-limited share of a cell (<= 1), 1.5e-6; bound 3e-6."""
+import numpy as np
+import pytest
+
+import helpers as H
+from mosegpu import abi
+
+pytestmark = pytest.mark.gpu
+
+SIZES = [(31, 7, 3), (32, 8, 4), (33, 9, 5), (34, 15, 2), (63, 16, 3), (65, 17, 1), (5, 41, 3)]
+
+
+@pytest.fixture(scope="module")
+def engine():
+    torch = pytest.importorskip("torch")
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from mosegpu.engine import Engine
+    return Engine
+
+
+def _steps(engine, case, precision, tol, exact=False, n=2):
+    import oracle
+    orc = oracle.Oracle(case)
+    P = case.P0.copy()
+    assert orc.step(P, n) == 0
+    eng = engine(case, precision=precision)
+    eng.step(n, graph=True)
+    m = case.interior_mask()
+    if exact:
+        assert np.array_equal(eng.state()[:, m], P[:, m])
+    e = H.rel_err(H.conserved(case, eng.state()), H.conserved(case, P))
+    assert np.all(e <= tol), e
+    assert eng.status().code == 0
+    eng.close()
+
+
+@pytest.mark.parametrize("riemann,limiter", [(abi.RS_HLLC, abi.LIM_MINMOD), (abi.RS_AUSMP, abi.LIM_VANLEER),
+                                             (abi.RS_LMROE, abi.LIM_VANALBADA), (abi.RS_LMROE, abi.LIM_MC),
+                                             (abi.RS_HLLC, abi.LIM_SUPERBEE), (abi.RS_AUSMP, abi.LIM_FIRST)])
+@pytest.mark.parametrize("n", SIZES)
+def test_duct_at_tile_edges(engine, n, riemann, limiter):
+    from mosegpu import case as cs
+    case = cs.duct_3d(widths=(n[0],), heights=(n[1],), depths=(n[2],), mach=1.5, amp=0.02, cfl=0.2, riemann=riemann,
+                      limiter=limiter, bc={2: abi.BC_EXTRAPOLATION, 3: abi.BC_WALL, 4: abi.BC_SYMMETRY,
+                                           5: abi.BC_EXTRAPOLATION, 6: abi.BC_EXTRAPOLATION})
+    _steps(engine, case, abi.PREC_FP64_FAST, 1e-12)
+    _steps(engine, case, abi.PREC_MIXED, 3e-6)
+
+
+@pytest.mark.parametrize("n", [(2, 2, 2), (3, 2, 4), (33, 9, 2), (4, 33, 3)])
+@pytest.mark.parametrize("mco", [1.0, 0.2])
+def test_two_cell_periodic_blocks(engine, n, mco):
+    """Connections whose donors are two cells deep (the one-launch fill copies both of their layers)."""
+    from mosegpu import case as cs
+    th = cs.ideal_gas_tables(mu=2e-2)
+    h = [1.0 / q for q in n]
+
+    def nodes(iu, iv, iw):
+        return np.stack([iu * h[0], iv * h[1], iw * h[2]], axis=-1)
+
+    def prim(c):
+        x, y, z = (2 * np.pi * c[..., q] for q in range(3))
+        return np.stack([1.0 + 0.1 * np.sin(x) * np.cos(y), 30 * np.sin(y) * np.cos(z), 20 * np.cos(x + z), 10 * np.sin(x),
+                         8.0e4 + 2e3 * np.cos(y + z)])
+    sch = dict(limiter=abi.LIM_VANALBADA, riemann=abi.RS_LMROE, visc=1, n_rk=3, ndir=3, cfl=0.4, prandtl=0.71, mco=mco,
+               dt_additive=1)
+    case = cs.layout_case("periodic", [[0, q] for q in n], nodes, (True,) * 3, {}, th, sch, prim)
+    _steps(engine, case, abi.PREC_FP64, 1e-12, exact=True)
+    _steps(engine, case, abi.PREC_FP64_FAST, 1e-12)
+
+
+BCS = {"wall": abi.BC_WALL, "extrapolation": abi.BC_EXTRAPOLATION, "symmetry": abi.BC_SYMMETRY, "none": abi.BC_NONE}
+
+
+@pytest.mark.parametrize("visc", [0, 1])
+@pytest.mark.parametrize("n2", [1, 2, 3])
+@pytest.mark.parametrize("low,high", [("wall", "wall"), ("wall", "extrapolation"), ("symmetry", "extrapolation"),
+                                      ("extrapolation", "extrapolation"), ("symmetry", "none")])
+def test_thin_axes_take_the_general_fill(engine, low, high, n2, visc):
+    """The rules that merge the ghost passes, and the records with them, against the sequential fill of the oracle: every
+    pair of face types on an axis of one, two and three cells, bit for bit."""
+    from mosegpu import case as cs
+    case = cs.multiblock_2d(cols=2, rows=1, widths=[6, 35], heights=[n2], visc=visc, mach=0.5, n_rk=3, cfl=0.2,
+                            riemann=abi.RS_HLLC, limiter=abi.LIM_MINMOD,
+                            bc={1: abi.BC_INFLOW, 2: abi.BC_EXTRAPOLATION, 3: BCS[low], 4: BCS[high],
+                                5: abi.BC_EXTRAPOLATION, 6: abi.BC_EXTRAPOLATION})
+    import oracle
+    orc = oracle.Oracle(case)
+    P = case.P0.copy()
+    if orc.step(P, 2) != 0:
+        pytest.skip("viscous faces one or two cells apart: the field leaves the tables in the oracle itself")
+    eng = engine(case)
+    eng.step(2, graph=True)
+    m = case.interior_mask()
+    assert np.array_equal(eng.state()[:, m], P[:, m])
+
+
+@pytest.mark.parametrize("nb,riemann", [(1, abi.RS_LMROE), (2, abi.RS_HLLC)])
+def test_autotuned_mixed_form_agrees(engine, nb, riemann):
+    """Whatever mb_autotune picks of the mixed 3-D sweep (chunk, queue, staging, CTAs per SM) gives the untuned result to
+    the rounding of the staged pressure (one FP32 ulp of p, 6e-8, in the faces of three stages and two steps; the bound
+    of the staging test, 1e-6, max-norm of the conserved variables, momentum against its vector)."""
+    from mosegpu import case as cs
+    case = cs.taylor_green(n=64, blocks=nb, riemann=riemann, share_geometry=nb > 1)
+    a, b = engine(case, precision=abi.PREC_MIXED), engine(case, precision=abi.PREC_MIXED)
+    b.fill_ghosts()
+    b.autotune()
+    a.step(2, graph=True)
+    b.step(2, graph=True)
+    e = H.rel_err(H.conserved(case, a.state()), H.conserved(case, b.state()))
+    assert np.all(e < 1e-6), e
