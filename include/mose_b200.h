@@ -447,8 +447,8 @@ int mb_read_group_status(mb_ctx* ctx, int g0, int n, mb_status* out, void* strea
 
 /* The sweep's autotuner (no counterpart in the reference): times, on the state P and the current mesh, the
  * k-chunk of the tiles of 3-D blocks (8 / 16 / 32 / 64 planes) and a plain grid (one CTA per tile) against the
- * persistent work queue (one wave of CTAs taking the largest tiles first from a counter), and keeps the
- * fastest for every later sweep. Does not change P or the clocks; call between steps. */
+ * persistent work queue (one wave of CTAs taking the largest tiles first from a counter), in the mixed form the
+ * staging and 3 or 4 CTAs per SM for 3-D tiles, and keeps the fastest for every later sweep. Does not change P or the clocks; call between steps. */
 int mb_autotune(mb_ctx* ctx, const double* P, void* stream);
 
 /* Sets the sweep configuration by hand: the k-chunk of 3-D tiles and the persistent work queue (1) or the plain
