@@ -31,7 +31,9 @@ struct DTile {
 // launch (pdl_next) and, before it touches anything an earlier kernel wrote, waits until the one before has ended and
 // its writes are visible (pdl_wait; every thread of every kernel of the chain, so that the end of one kernel implies the
 // end of all before it). What it does before the wait reads only the mesh tables, which no kernel writes. Only
-// on the smallest meshes (Params::chain).
+// on the smallest meshes (Params::chain). Since such a kernel may run before its input is written, the arrays that kernels
+// write (state arenas, Ur, local steps) are read by ordinary loads, here and in all these kernels call: ld() and const
+// __restrict__ parameters take the read-only path, which is for data that holds for a kernel's whole life.
 __device__ __forceinline__ void pdl_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
@@ -141,8 +143,8 @@ MB_HD void face_flux(const Params& p, const DBlk& b, const Tile<R, TY, NVT, KM>&
   }
   R urL = (R)0, urR = (R)0;
   if (RS == 0 && p.prec) {  // HLLC-PC: the Ur of the face's two cells (conv_physics.inc:159-163)
-    urL = (R)ld(p.ur + b.boff + l0);
-    urR = (R)ld(p.ur + b.boff + l0 + st);
+    urL = (R)p.ur[b.boff + l0];
+    urR = (R)p.ur[b.boff + l0 + st];
   }
   conv_face<R, RS, LIM>(p, pm1, p0, pp1, pp2, dlc, nx, ny, nz, area, out, bet, urL, urR);
   if (!VISC) return;
@@ -228,8 +230,7 @@ MB_HD void bc_face_geom(const DBlk& b, int Im, int Jm, int Km, int F, double* g)
 
 // BC_Connection_Eul_lean (Lib_BC.f90:1770-1867)
 template <typename R, int RS = 0, int LIM = 0>
-MB_HD void bc_conn_eul(const Params& p, const DBlk& b, const double* __restrict__ P, int Im, int Jm,
-                                         int Km, int Fm, R* A) {
+MB_HD void bc_conn_eul(const Params& p, const DBlk& b, const double* P, int Im, int Jm, int Km, int Fm, R* A) {
   const long long nc = p.nc;
   const int rs = RS ? RS : p.rs;
   const int lim = LIM ? LIM : p.lim;
@@ -254,17 +255,16 @@ MB_HD void bc_conn_eul(const Params& p, const DBlk& b, const double* __restrict_
                           // its k = 1 cells
     const double* pp = P + MB_IPR * nc;
     const long long sj = b.pi, sk = b.kmirror ? 0 : (long long)b.pi * b.pj;
-    beta_ = sd_beta<R>(p.sd, cvt<R>(ld(pp + rm)), cvt<R>(ld(pp + rm - 1)), cvt<R>(ld(pp + rm + 1)),
-                       cvt<R>(ld(pp + rm - sj)), cvt<R>(ld(pp + rm + sj)), cvt<R>(ld(pp + rm - sk)),
-                       cvt<R>(ld(pp + rm + sk)));
+    beta_ = sd_beta<R>(p.sd, cvt<R>(pp[rm]), cvt<R>(pp[rm - 1]), cvt<R>(pp[rm + 1]), cvt<R>(pp[rm - sj]),
+                       cvt<R>(pp[rm + sj]), cvt<R>(pp[rm - sk]), cvt<R>(pp[rm + sk]));
   }
   R Dl1 = dlc4[0] * (R)0.5, Dl2 = dlc4[1] * (R)0.5, Dl3 = dlc4[2] * (R)0.5, Dl4 = dlc4[3] * (R)0.5;
   R D12 = Dl1 + Dl2, D23 = Dl2 + Dl3, D34 = Dl3 + Dl4;
   R PL[MB_NP], PR[MB_NP];
 #pragma unroll
   for (int s = 0; s < MB_NP; ++s) {
-    R q1 = cvt<R>(ld(P + rr[0] + s * nc)), q2 = cvt<R>(ld(P + rr[1] + s * nc)), q3 = cvt<R>(ld(P + rr[2] + s * nc)),
-      q4 = cvt<R>(ld(P + rr[3] + s * nc));
+    R q1 = cvt<R>(P[rr[0] + s * nc]), q2 = cvt<R>(P[rr[1] + s * nc]), q3 = cvt<R>(P[rr[2] + s * nc]),
+      q4 = cvt<R>(P[rr[3] + s * nc]);
     R d21 = (q2 - q1) / D12, d32 = (q3 - q2) / D23, d43 = (q4 - q3) / D34;
     PL[s] = q2 + beta_ * rlimiter(lim, d32, d21) * Dl2;
     PR[s] = q3 - beta_ * rlimiter(lim, d43, d32) * Dl3;
@@ -276,7 +276,7 @@ MB_HD void bc_conn_eul(const Params& p, const DBlk& b, const double* __restrict_
   R aR = f_ss(p, PR[0], PR[MB_IPR], rhoR, RRr);
   R F_r, F_u, F_v, F_w, F_E;
   // HLLC-PC: the Ur of cells 2 and 3, the ghost's 0 (never filled, Lib_BC.f90:1739-1742)
-  const R urL = (RS == 0 && p.prec) ? (R)ld(p.ur + rr[1]) : (R)0, urR = (RS == 0 && p.prec) ? (R)ld(p.ur + rr[2]) : (R)0;
+  const R urL = (RS == 0 && p.prec) ? (R)p.ur[rr[1]] : (R)0, urR = (RS == 0 && p.prec) ? (R)p.ur[rr[2]] : (R)0;
   riemann_rec<R, RS>(p, PL[0], PL[MB_IU], PL[MB_IV], PL[MB_IW], PL[MB_IPR], aL, rhoL, RL, PR[0], PR[MB_IU], PR[MB_IV],
                      PR[MB_IW], PR[MB_IPR], aR, rhoR, RRr, nx, ny, nz, F_r, F_u, F_v, F_w, F_E, beta_, urL, urR);
   R su = copysign((R)0.5, F_r), selL = (R)0.5 + su, selR = su - (R)0.5;
@@ -294,7 +294,7 @@ MB_HD void bc_conn_eul(const Params& p, const DBlk& b, const double* __restrict_
 // filled state, so this reads those cells of P in place: pgr = the six donor rows of the record (the same values,
 // without the copy pass and its nconn x 30 FP64 buffer).
 template <typename R>
-MB_HD void bc_conn_visc(const Params& p, const DBlk& b, const double* __restrict__ P, int Im, int Jm,
+MB_HD void bc_conn_visc(const Params& p, const DBlk& b, const double* P, int Im, int Jm,
                                           int Km, int Fm, const long long* __restrict__ pgr, R* S) {
   const long long nc = p.nc;
   int dir = (Fm + 1) / 2, modfm2 = 1 - 2 * (Fm % 2), gstep = 2 * (Fm % 2) - 1;
@@ -317,9 +317,9 @@ MB_HD void bc_conn_visc(const Params& p, const DBlk& b, const double* __restrict
   const long long scm = (b.kmirror && ic == 2) ? 0 : sc;  // a mirrored block's k ghosts are its k = 1 cells
   const long long rc[6] = {r1, 0, r1 + sb, r1 - sb, r1 + scm, r1 - scm};
   auto pv = [&](int q, int s) -> R {
-    if (q == 1) return cvt<R>(ld(P + pgr[0] + s * nc));
-    if (q >= 6) return cvt<R>(ld(P + pgr[q - 4] + s * nc));
-    return cvt<R>(ld(P + rc[q] + s * nc));
+    if (q == 1) return cvt<R>(P[pgr[0] + s * nc]);
+    if (q >= 6) return cvt<R>(P[pgr[q - 4] + s * nc]);
+    return cvt<R>(P[rc[q] + s * nc]);
   };
   R rh[10], rg[10];
 #pragma unroll
@@ -364,13 +364,13 @@ MB_HD void bc_conn_visc(const Params& p, const DBlk& b, const double* __restrict
 
 // BC_Extrapolation (Lib_BC.f90:1119-1165)
 template <typename R>
-MB_HD void bc_extrap(const Params& p, const DBlk& b, const double* __restrict__ P, int Im, int Jm,
+MB_HD void bc_extrap(const Params& p, const DBlk& b, const double* P, int Im, int Jm,
                                        int Km, int Fm, R* A) {
   const long long nc = p.nc;
   const long long r = row(b, Im, Jm, Km);
   R Pr[MB_NP];
 #pragma unroll
-  for (int s = 0; s < MB_NP; ++s) Pr[s] = cvt<R>(ld(P + r + s * nc));
+  for (int s = 0; s < MB_NP; ++s) Pr[s] = cvt<R>(P[r + s * nc]);
   double g[4];
   bc_face_geom(b, Im, Jm, Km, Fm, g);
   R nx = cvt<R>(g[0]), ny = cvt<R>(g[1]), nz = cvt<R>(g[2]), area = cvt<R>(g[3]);
@@ -393,7 +393,7 @@ MB_HD void bc_extrap(const Params& p, const DBlk& b, const double* __restrict__ 
 // reconstruction, Riemann problem between the face state and its mirror; momentum rows only. The Euler part of
 // the adiabatic wall and the closed-inlet fallback of the 405 record.
 template <typename R, int RS = 0, int LIM = 0>
-MB_HD void bc_sym_eul(const Params& p, const DBlk& b, const double* __restrict__ P, int Im, int Jm, int Km,
+MB_HD void bc_sym_eul(const Params& p, const DBlk& b, const double* P, int Im, int Jm, int Km,
                                int Fm, R* A) {
   const long long nc = p.nc;
   const int lim = LIM ? LIM : p.lim;
@@ -408,7 +408,7 @@ MB_HD void bc_sym_eul(const Params& p, const DBlk& b, const double* __restrict__
   R Int_Dl = (R)0.5 * cvt<R>(ld(b.dl + (dir - 1) + 3 * (ri - b.boff)));
   R B[MB_NP], I[MB_NP], G[MB_NP], F[MB_NP];
 #pragma unroll
-  for (int s = 0; s < MB_NP; ++s) { B[s] = cvt<R>(ld(P + rb + s * nc)); I[s] = cvt<R>(ld(P + ri + s * nc)); }
+  for (int s = 0; s < MB_NP; ++s) { B[s] = cvt<R>(P[rb + s * nc]); I[s] = cvt<R>(P[ri + s * nc]); }
   R Un = B[MB_IU] * nrm[0] + B[MB_IV] * nrm[1] + B[MB_IW] * nrm[2];
 #pragma unroll
   for (int s = 0; s < MB_NP; ++s) G[s] = B[s];
@@ -437,7 +437,7 @@ MB_HD void bc_sym_eul(const Params& p, const DBlk& b, const double* __restrict__
 #pragma unroll
   for (int a = 0; a < 3; ++a) { U1[a] = Un1 * nrm[a] + Vt[a]; U4[a] = -Un1 * nrm[a] + Vt[a]; }
   R F_r, F_u, F_v, F_w, F_E;
-  const R urc = (RS == 0 && p.prec) ? (R)ld(p.ur + rb) : (R)0;  // HLLC-PC: the cell's Ur on both sides (:720-723)
+  const R urc = (RS == 0 && p.prec) ? (R)p.ur[rb] : (R)0;  // HLLC-PC: the cell's Ur on both sides (:720-723)
   riemann_rec<R, RS>(p, F[0], U1[0], U1[1], U1[2], F[MB_IPR], Sound, rotot, Rtot, F[0], U4[0], U4[1], U4[2],
                      F[MB_IPR], Sound, rotot, Rtot, nrm[0], nrm[1], nrm[2], F_r, F_u, F_v, F_w, F_E, (R)1, urc, urc);
   A[0] = (R)-0.0;  // an exact no-op when added: only the momentum rows change
@@ -450,14 +450,14 @@ MB_HD void bc_sym_eul(const Params& p, const DBlk& b, const double* __restrict__
 // BC_Wall_Heat_dev (Lib_BC.f90:879-982), laminar adiabatic no-slip wall: the wall-normal velocity gradient of the
 // boundary cell, Grad . M of the cell, Stress_Vector_Std (Mod_Fluid.f90:20-44) with mu_t = 0; momentum rows only.
 template <typename R>
-MB_HD void bc_wall_heat(const Params& p, const DBlk& b, const double* __restrict__ P, int Im, int Jm, int Km,
+MB_HD void bc_wall_heat(const Params& p, const DBlk& b, const double* P, int Im, int Jm, int Km,
                                  int Fm, R* S) {
   const long long nc = p.nc;
   int dir = (Fm + 1) / 2, modfm = Fm % 2, modfm2 = 1 - 2 * modfm, modfm3 = 2 * (2 * modfm - 1);
   const long long rb = row(b, Im, Jm, Km), l = rb - b.boff;
   R Pb[MB_NP];
 #pragma unroll
-  for (int s = 0; s < MB_NP; ++s) Pb[s] = cvt<R>(ld(P + rb + s * nc));
+  for (int s = 0; s < MB_NP; ++s) Pb[s] = cvt<R>(P[rb + s * nc]);
   R M[3][3];
 #pragma unroll
   for (int a = 0; a < 3; ++a)
@@ -519,14 +519,14 @@ MB_HD void stress_std(const R G2[3][3], R nx, R ny, R nz, R mil, R* S) {
 // the face give the normal and transverse velocity gradients; the stress of Grad . M (momentum rows) and its work on
 // the face-mean velocity (energy row), subtracted.
 template <typename R>
-MB_HD void bc_sym_visc(const Params& p, const DBlk& b, const double* __restrict__ P, int Im, int Jm, int Km, int Fm,
+MB_HD void bc_sym_visc(const Params& p, const DBlk& b, const double* P, int Im, int Jm, int Km, int Fm,
                        R* S) {
   const long long nc = p.nc;
   const int modfm = Fm % 2, modfm2 = 1 - 2 * modfm;
   const long long rb = row(b, Im, Jm, Km), l = rb - b.boff;
   R Pb[MB_NP];
 #pragma unroll
-  for (int s = 0; s < MB_NP; ++s) Pb[s] = cvt<R>(ld(P + rb + s * nc));
+  for (int s = 0; s < MB_NP; ++s) Pb[s] = cvt<R>(P[rb + s * nc]);
   R M[3][3];
 #pragma unroll
   for (int a = 0; a < 3; ++a)
@@ -546,10 +546,10 @@ MB_HD void bc_sym_visc(const Params& p, const DBlk& b, const double* __restrict_
   R V1[3] = {Pb[MB_IU], Pb[MB_IV], Pb[MB_IW]}, V3[3], V4[3], V7[3], V8[3];
 #pragma unroll
   for (int q = 0; q < 3; ++q) {
-    V3[q] = cvt<R>(ld(P + rb - sb + (MB_IU + q) * nc));
-    V4[q] = cvt<R>(ld(P + rb + sb + (MB_IU + q) * nc));
-    V7[q] = cvt<R>(ld(P + rb - sc + (MB_IU + q) * nc));
-    V8[q] = cvt<R>(ld(P + rb + sc + (MB_IU + q) * nc));
+    V3[q] = cvt<R>(P[rb - sb + (MB_IU + q) * nc]);
+    V4[q] = cvt<R>(P[rb + sb + (MB_IU + q) * nc]);
+    V7[q] = cvt<R>(P[rb - sc + (MB_IU + q) * nc]);
+    V8[q] = cvt<R>(P[rb + sc + (MB_IU + q) * nc]);
   }
   double g[4];
   bc_face_geom(b, Im, Jm, Km, Fm, g);
@@ -592,7 +592,7 @@ MB_HD void bc_sym_visc(const Params& p, const DBlk& b, const double* __restrict_
 // (p of the cell at T_wall; k = mu cp / Pr when Pr > 0), the wall-normal velocity and temperature gradients of the
 // boundary cell: stress (momentum rows) and conducted heat (energy row), subtracted.
 template <typename R>
-MB_HD void bc_wall_temp(const Params& p, const DBlk& b, const double* __restrict__ P, int Im, int Jm, int Km, int Fm,
+MB_HD void bc_wall_temp(const Params& p, const DBlk& b, const double* P, int Im, int Jm, int Km, int Fm,
                         double Tw_, R* S) {
   const long long nc = p.nc;
   int dir = (Fm + 1) / 2, modfm = Fm % 2, modfm2 = 1 - 2 * modfm, modfm3 = 2 * (2 * modfm - 1);
@@ -600,7 +600,7 @@ MB_HD void bc_wall_temp(const Params& p, const DBlk& b, const double* __restrict
   const R Tw = cvt<R>(Tw_);
   R Pb[MB_NP];
 #pragma unroll
-  for (int s = 0; s < MB_NP; ++s) Pb[s] = cvt<R>(ld(P + rb + s * nc));
+  for (int s = 0; s < MB_NP; ++s) Pb[s] = cvt<R>(P[rb + s * nc]);
   R M[3][3];
 #pragma unroll
   for (int a = 0; a < 3; ++a)
@@ -790,7 +790,7 @@ MB_HD void subsonic_inflow_face(const Params& p, const R* Bp, R Un, R Sound, R G
 // inlet face (BC_Symmetry_Eul) or leaves to pamb (BC_Outflow, 407); inward flow takes the supersonic static inlet
 // (405, or mach > 1: BC_Supersonic_Inflow, Lib_BC.f90:1247-1330) or the subsonic closure (BC_Subsonic_Inflow).
 template <typename R, int RS = 0, int LIM = 0>
-MB_HD void bc_inflow(const Params& p, const DBlk& b, const double* __restrict__ P, int Im, int Jm, int Km,
+MB_HD void bc_inflow(const Params& p, const DBlk& b, const double* P, int Im, int Jm, int Km,
                               int Fm, const double* __restrict__ q, R* A) {
   const long long nc = p.nc;
   const int lim = LIM ? LIM : p.lim;
@@ -799,7 +799,7 @@ MB_HD void bc_inflow(const Params& p, const DBlk& b, const double* __restrict__ 
   const long long rb = row(b, Im, Jm, Km), ri = rb + gstep * st;
   R P2[MB_NP], Ip[MB_NP];
 #pragma unroll
-  for (int s = 0; s < MB_NP; ++s) { P2[s] = cvt<R>(ld(P + rb + s * nc)); Ip[s] = cvt<R>(ld(P + ri + s * nc)); }
+  for (int s = 0; s < MB_NP; ++s) { P2[s] = cvt<R>(P[rb + s * nc]); Ip[s] = cvt<R>(P[ri + s * nc]); }
   double g[4];
   bc_face_geom(b, Im, Jm, Km, Fm, g);
   R nx = cvt<R>(g[0]), ny = cvt<R>(g[1]), nz = cvt<R>(g[2]), area = cvt<R>(g[3]);
@@ -900,14 +900,14 @@ MB_HD void bc_inflow(const Params& p, const DBlk& b, const double* __restrict__ 
 // (BC_Symmetry_Eul); otherwise the face state of BC_Outflow (Lib_BC.f90:1166-1240) from the Riemann invariant towards
 // the face and the relaxed exit pressure (isentropic when the normal Mach number is below 1 and p_exit > 0).
 template <typename R, int RS = 0, int LIM = 0>
-MB_HD void bc_outlet(const Params& p, const DBlk& b, const double* __restrict__ P, int Im, int Jm, int Km, int Fm,
+MB_HD void bc_outlet(const Params& p, const DBlk& b, const double* P, int Im, int Jm, int Km, int Fm,
                      const double* __restrict__ q, R* A) {
   const long long nc = p.nc;
   const int modfm = Fm % 2, modfm2 = 1 - 2 * modfm;
   const long long rb = row(b, Im, Jm, Km);
   R Bp[MB_NP];
 #pragma unroll
-  for (int s = 0; s < MB_NP; ++s) Bp[s] = cvt<R>(ld(P + rb + s * nc));
+  for (int s = 0; s < MB_NP; ++s) Bp[s] = cvt<R>(P[rb + s * nc]);
   double g[4];
   bc_face_geom(b, Im, Jm, Km, Fm, g);
   const R nrm[3] = {cvt<R>(g[0]), cvt<R>(g[1]), cvt<R>(g[2])};
@@ -947,7 +947,7 @@ MB_HD int record_of(const Params& p, const DBlk& b, int F, int i, int j, int k) 
 // and then, in Navier-Stokes, S is subtracted (the order of the reference's statements); components a record leaves
 // alone hold exact no-ops (-0 in A, +0 in S).
 template <typename R, bool VISC, int RS = 0, int LIM = 0>
-MB_HD void bc_record(const Params& p, const DBlk& b, const double* __restrict__ P, int rid, int i, int j, int k, int F,
+MB_HD void bc_record(const Params& p, const DBlk& b, const double* P, int rid, int i, int j, int k, int F,
                      R* A, R* S) {
   const DRec& rc = p.rec[rid];
   if (VISC)
@@ -1076,7 +1076,7 @@ __device__ __forceinline__ void clock_groups(const Params& p) {
 // VAR tells apart the instantiations of the same types built with different flags (the FP64 production form's units)
 template <typename R, bool VISC, int RS, int LIM, int VAR = 0>
 __global__ void __launch_bounds__(128) k_records(Params p, const RecWork* __restrict__ work, int nrec,
-                                               const double* __restrict__ P, Surface sf) {
+                                               const double* P, Surface sf) {
   pdl_next();
   const int nbr = (nrec + 127) / 128;
   if ((int)blockIdx.x >= nbr) {  // the ghosts and the clock (meshes whose records read no ghost)
@@ -1569,7 +1569,7 @@ __device__ __forceinline__ void put_cell(const Params& p, const Tile<R, TY, NVT,
 }
 
 template <typename R, int TY, int NVT, bool KM>
-__device__ __forceinline__ void stage_plane(const Params& p, const DBlk& b, const double* __restrict__ P,
+__device__ __forceinline__ void stage_plane(const Params& p, const DBlk& b, const double* P,
                                             const Tile<R, TY, NVT, KM>& T, int i0, int j0, int kk, int jext) {
   const int sl = slot_of<KM>(kk);
   const long long nc = p.nc;
@@ -1581,7 +1581,7 @@ __device__ __forceinline__ void stage_plane(const Params& p, const DBlk& b, cons
     if (i >= 1 - GC && i <= b.n1 + GC && j >= 1 - jext && j <= b.n2 + jext) {
       const long long r = row(b, i, j, kk);
 #pragma unroll
-      for (int s = 0; s < MB_NP; ++s) vals[s] = cvt<R>(ld(P + r + s * nc));
+      for (int s = 0; s < MB_NP; ++s) vals[s] = cvt<R>(P[r + s * nc]);
       put_cell<R, TY, NVT, KM>(p, T, o, vals);
     } else {
       T.put(o, (R)0, (R)0, (R)0, (R)0, (R)0, (R)0);
@@ -1682,7 +1682,7 @@ __device__ __forceinline__ void stage_plane_raw(const Params& p, const DBlk& b, 
 // With TMA staging (the mixed form, p.tmap set) raw is the staging buffer and bar its mbarrier, phase the parity the
 // CTA waits for next; false: a bounded wait gave up (the clock's code is set to MB_E_TIMEOUT) and the CTA must stop.
 template <typename R, int TY, bool VISC, int MODE, int RS, int LIM, bool KM, int STG>
-__device__ __forceinline__ bool sweep_tile(const Params& p, const DTile t, const double* __restrict__ Pin,
+__device__ __forceinline__ bool sweep_tile(const Params& p, const DTile t, const double* Pin,
                                            const double* Pold, double* Pout, double* Rout, double rkc, int last,
                                            unsigned char* smem_raw, double* sred, double* s_res, TmaStage& ts,
                                            DBlk& sblk) {
@@ -1968,7 +1968,7 @@ __device__ __forceinline__ bool sweep_tile(const Params& p, const DTile t, const
       } else {
         double pc[MB_NP], po[MB_NP], pn[MB_NP];
 #pragma unroll
-        for (int s = 0; s < MB_NP; ++s) pc[s] = ld(Pin + r + s * p.nc);
+        for (int s = 0; s < MB_NP; ++s) pc[s] = Pin[r + s * p.nc];
 #pragma unroll
         for (int s = 0; s < MB_NP; ++s) po[s] = Pold[r + s * p.nc];
         double rho, Tc, irho = 0.0;
@@ -1987,14 +1987,14 @@ __device__ __forceinline__ bool sweep_tile(const Params& p, const DTile t, const
         const double vol = ld(b.vol + (r - b.boff));
         double dtc = dt;
         if (RS == 0 && p.prec) {
-          dtc = ld(p.dtl + r) * st->rampf;  // the steps of the start of the step (Ur of that state)
+          dtc = p.dtl[r] * st->rampf;  // the steps of the start of the step (Ur of that state)
         } else if (RS == 0 && p.local_dt) {  // the cell's own step in the flux type (FP64 in the parity form)
           R pr[MB_NP];
 #pragma unroll
           for (int s = 0; s < MB_NP; ++s) pr[s] = cvt<R>(po[s]);
           dtc = (double)cell_dt_t<R>(p, b, r - b.boff, pr) * st->rampf;
         }
-        if (RS == 0 && p.intvar) prim_update(p, pc, po, acc, vol, dtc, rkc, pn, p.prec ? ld(p.ur + r) : 0.0);
+        if (RS == 0 && p.intvar) prim_update(p, pc, po, acc, vol, dtc, rkc, pn, p.prec ? p.ur[r] : 0.0);
         else if (Fast<R>::on) cons_update_fast(p, pc, po, acc, vol, dtc, rkc, irho, Tl, Tc, pn, r);
         else cons_update(p, pc, po, acc, vol, dtc, rkc, Tc, pn, r);
         bool bad = !(pn[MB_IPR] >= 0.0);
@@ -2071,7 +2071,7 @@ MB_HD constexpr size_t sweep_smem() {
 template <typename R, int TY, bool VISC, int MODE, int RS, int LIM, int MINB, bool KM = false, int VAR = 0,
           int STG = STG_PLAIN>
 __global__ void __launch_bounds__(32 * TY, MINB)
-k_sweep(Params p, const DTile* __restrict__ tiles, const double* __restrict__ Pin, const double* Pold, double* Pout,
+k_sweep(Params p, const DTile* __restrict__ tiles, const double* Pin, const double* Pold, double* Pout,
         double* Rout, double rkc, int last) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ double sred[32];

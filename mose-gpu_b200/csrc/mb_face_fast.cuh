@@ -418,8 +418,7 @@ struct ArenaCells {
   R iri;
   bool low;                // the boundary cell is the upper one (a low face)
   __device__ __forceinline__ void uvwT(long long r, V2<R>& A, V2<R>& B, V2<R>& C) const {
-    const R rho = (R)ld(P + r), u = (R)ld(P + r + nc), v = (R)ld(P + r + 2 * nc), w = (R)ld(P + r + 3 * nc),
-            pr = (R)ld(P + r + 4 * nc);
+    const R rho = (R)P[r], u = (R)P[r + nc], v = (R)P[r + 2 * nc], w = (R)P[r + 3 * nc], pr = (R)P[r + 4 * nc];
     A = mk2<R>(u, v);
     B = mk2<R>(w, pr * iri * rcp_(rho));
     C = mk2<R>(rho, pr);
@@ -439,7 +438,7 @@ struct ArenaCells {
 // two viscous fluxes the reference averages, with the gradients of the cell and of its ghost, are one flux with the
 // mean gradient (the flux is linear in it): the interior face's.
 template <typename R, bool VISC, int RS, int LIM>
-__device__ __forceinline__ void conn_fast(const Params& p, const DBlk& b, const double* __restrict__ P, int i, int j,
+__device__ __forceinline__ void conn_fast(const Params& p, const DBlk& b, const double* P, int i, int j,
                                           int k, int F, const long long* __restrict__ pg, R* out) {
   const int d = (F - 1) >> 1, low = F & 1;
   const int gst = (d == 0) ? 1 : (d == 1 ? b.pi : b.pi * b.pj);

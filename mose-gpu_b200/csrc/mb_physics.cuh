@@ -239,6 +239,7 @@ MB_HD int fmi32(const DBlk& b, int d, int i, int j, int k) {
   if (d == 1) return 4 * ((i - 1) + b.n1 * (j + (b.n2 + 1) * (k - 1)));
   return 4 * ((i - 1) + b.n1 * ((j - 1) + b.n2 * k));
 }
+// a value of a table that no kernel writes (geometry, gas tables, record parameters): the read-only path
 MB_HD double ld(const double* p) { return ldg_(p); }
 MB_HD float ld(const float* p) { return ldg_(p); }
 
