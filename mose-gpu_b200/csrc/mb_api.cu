@@ -1298,7 +1298,8 @@ static int stage_compute(mb_ctx* c, const double* in, const double* P, double* o
   return MB_OK;
 }
 
-// the clock of a step can be advanced by the first stage's ghost fill: nothing in that launch reads it
+// the clock of a step can be advanced by the first stage's ghost fill: nothing in that launch reads it (the records that
+// share the launch leave out their test of the case's done flag)
 static bool clock_in_fill(const mb_ctx* c) { return c->gf.fused && !c->p.prec; }
 
 // clock: the stage also advances the case clocks, before its sweep (only where clock_in_fill)

@@ -1096,7 +1096,9 @@ __global__ void __launch_bounds__(128) k_records(Params p, const RecWork* __rest
   if (q >= nrec) return;
   const int rid = w1.z, face = w1.x, type = w1.y;
   const DBlk& b = p.blk[w0.x];
-  if (p.st[b.grp].done) return;
+  // Where the clock shares the launch it may be setting the flag now, so its records are computed whatever the flag says
+  // (those of a case that has just ended are not read: its tiles return).
+  if (!sf.clock && p.st[b.grp].done) return;
   if constexpr (Fast<R>::on && RS != 0) {
     R v[MB_NP];
     if (type == 1) {

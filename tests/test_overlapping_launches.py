@@ -35,3 +35,18 @@ def test_the_looked_for_names_are_the_ones_in_use():
     assert set(re.findall(r"double\s*\*\s*(\w+)", args)) <= {"Pin", "Pold", "Pout", "Rout"}
     args = re.search(r"k_records\((.*?)\)\s*\{", s, re.S).group(1)
     assert set(re.findall(r"double\s*\*\s*(\w+)", args)) == {"P"}
+
+
+def test_the_records_do_not_read_what_the_clock_of_their_launch_writes():
+    """k_records may carry the case clocks in a block of its own: clock_groups writes the DevState of every case there, so
+    no other block of that launch reads one (the done flag only where the launch has no clock)."""
+    s = source("mb_engine.cuh")
+    body = s[s.index("k_records("):]
+    body = body[:body.index("\n}\n")]
+    reads = re.findall(r"[^;{}\n]*\bp\.st\b[^;\n]*", body)
+    assert reads and all("!sf.clock &&" in r for r in reads), reads
+    # the functions it calls for a record take nothing from the clocks
+    for name in HEADERS:
+        h = source(name)
+        for f in re.findall(r"MB_HD void (?:bc_\w+|conn_fast|ghost_record)\([^{]*\{.*?\n\}\n", h, re.S):
+            assert not re.search(r"\bp\.st\b|->time\b|->dt\b|rampf", f), f[:80]
