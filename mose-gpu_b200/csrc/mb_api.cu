@@ -587,8 +587,10 @@ static int build_tables(mb_ctx* c, const mb_mesh* mesh) {
   // one's ghosts (the reference fills them in one sequential record loop). Every record goes into the first half
   // unless its opposite partner on the same column comes earlier in record order; only pairs interact, so two
   // launches per pass reproduce the sequential order exactly. An axis of one cell with type 11 on both faces is
-  // order-free (every ghost equals the cell), as are axes of three or more cells.
+  // order-free (every ghost equals the cell), as are axes of three or more cells; with a record on one face only (lone)
+  // the cubic ghost reads what the caller put into the other face's ghosts.
   int ordered = 0;
+  bool lone = false;
   std::vector<char> late_phys(mesh->nrec, 0), late_cubic(mesh->nrec, 0);
   {
     std::vector<int> ax11(3 * (size_t)mesh->nblk, 1);
@@ -599,6 +601,12 @@ static int build_tables(mb_ctx* c, const mb_mesh* mesh) {
       const int ax = (r.face - 1) / 2, nax = mesh->blk[r.blk].n[ax];
       if (r.type != MB_BC_EXTRAPOLATION && r.type != MB_BC_WALL && r.type != MB_BC_WALL_T) continue;
       if (nax == 2 || (nax == 1 && !ax11[3 * r.blk + ax])) ordered = 1;
+      if (nax == 1) {  // the record of the same column on the opposite face
+        const DBlk& d = hb[r.blk];
+        const int m = d.rmap[(r.face - 1) ^ 1];
+        const int t = ax == 0 ? (r.j - 1) + (r.k - 1) * d.n2 : (ax == 1 ? (r.i - 1) + (r.k - 1) * d.n1 : (r.i - 1) + (r.j - 1) * d.n1);
+        if (m < 0 || recmap[m + t] < 0) lone = true;
+      }
     }
     if (ordered) {
       std::unordered_map<unsigned long long, int> seen_phys, seen_cubic;  // column -> face of its first record
@@ -656,7 +664,7 @@ static int build_tables(mb_ctx* c, const mb_mesh* mesh) {
   g.rec = c->d_grec; g.phys = c->d_phys; g.nphys = (int)phys.size(); g.cubic = c->d_cubic; g.ncubic = (int)cubic.size();
   g.cdst = c->d_cdst; g.csrc = c->d_csrc; g.ncopy = (int)cdst.size(); g.pgsrc = c->d_pgsrc; g.nconn = mesh->nconn;
   g.ordered = ordered;
-  g.fused = !ordered && deep_donors;
+  g.fused = !ordered && deep_donors && !lone;
   bool reads_ghosts = false;  // a record of the work list reads a ghost row
   for (const RecWork& w : work) {
     const int ax = (w.face - 1) / 2;

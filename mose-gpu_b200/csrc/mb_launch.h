@@ -23,8 +23,9 @@ struct GhostLists {
   // holding the records whose opposite-face partner on the same column comes earlier in record order; each pass then
   // runs as two launches (only on blocks with an axis of at most two cells does the order change values)
   int ordered;
-  // fused != 0: no ghost is computed from another ghost of the fill (ordered == 0, and every connection copies interior
-  // cells of its donor: the donor is at least two cells deep along its axis), so that one launch fills all of them
+  // fused != 0: no ghost is computed from another ghost (ordered == 0, a one-cell axis has a record on both of its faces,
+  // and every connection copies interior cells of its donor: the donor is at least two cells deep along its axis), so
+  // that one launch fills all of them
   int fused;
   // surface != 0: fused, and no boundary record reads a ghost (no connections, no viscous symmetry face, and two cells
   // along the axis where a record reads the cell behind the boundary cell), so that the stage's records, its ghost fill

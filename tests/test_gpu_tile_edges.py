@@ -117,3 +117,27 @@ def test_autotuned_mixed_form_agrees(engine, nb, riemann):
     b.step(2, graph=True)
     e = H.rel_err(H.conserved(case, a.state()), H.conserved(case, b.state()))
     assert np.all(e < 1e-6), e
+
+
+def test_a_one_cell_axis_with_a_condition_on_one_side_only(engine):
+    """A face without records keeps the ghosts its caller put there (a halo, say), and the cubic ghost of the opposite face
+    of a one-cell axis reads them: the sequential fill of the oracle, bit for bit. The records of one side, of the other,
+    and of half a side."""
+    from mosegpu import case as cs
+    import oracle
+    g = np.random.default_rng(5)
+    for keep in (lambda r: r["face"] != 4, lambda r: r["face"] != 3, lambda r: (r["face"] != 4) | (r["i"] > 17)):
+        case = cs.multiblock_2d(cols=1, rows=1, widths=[35], heights=[1], visc=1, mach=0.5, n_rk=3,
+                                riemann=abi.RS_HLLC, limiter=abi.LIM_MINMOD,
+                                bc={1: abi.BC_INFLOW, 2: abi.BC_EXTRAPOLATION, 3: abi.BC_EXTRAPOLATION,
+                                    4: abi.BC_EXTRAPOLATION, 5: abi.BC_EXTRAPOLATION, 6: abi.BC_EXTRAPOLATION})
+        assert len(case.conn) == 0
+        case.rec = case.rec[keep(case.rec)].copy()
+        inside = case.P0[:, case.interior_mask()].mean(axis=1, keepdims=True)
+        case.P0 = np.where(case.interior_mask()[None], case.P0, inside * (1.0 + 0.01 * g.standard_normal(case.P0.shape)))
+        P = case.P0.copy()
+        oracle.Oracle(case).fill_ghosts(P)
+        eng = engine(case)
+        eng.fill_ghosts()
+        assert np.array_equal(eng.state(), P)
+        eng.close()
