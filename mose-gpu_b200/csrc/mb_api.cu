@@ -57,7 +57,8 @@ struct mb_ctx {
   int persistent_km = 0;        // the same for the tiles of mirrored one-plane blocks (autotuned)
   float tuned_ms = 0.f;         // sweep time of the chosen configuration
   int* d_queue = nullptr;       // tile counter of the persistent sweep
-  int ty_sweep = 4;
+  int ty_sweep = 4;             // tile rows of the context's sweep unit, and of its one-plane tiles
+  int ty_km = 4;
   int nsm = 148;                // SMs of the device
   DTile* d_tiles_aux = nullptr;
   int ntiles_aux = 0;
@@ -523,9 +524,9 @@ static int build_tables(mb_ctx* c, const mb_mesh* mesh) {
     for (int q = 0; q < 4; ++q) c->kcls[q] = kc;
   }
   std::vector<DTile> ts = make_tiles(c->hdims, c->ty_sweep, c->kc3, 0xe, &c->hkm, 0, c->kcls);
-  std::vector<DTile> tk = make_tiles(c->hdims, c->ty_sweep, c->kc3, 0xe, &c->hkm, 1);
+  std::vector<DTile> tk = make_tiles(c->hdims, c->ty_km, c->kc3, 0xe, &c->hkm, 1);
   if (c->persistent) sort_by_work(ts, c->hdims, c->ty_sweep);
-  if (c->persistent_km) sort_by_work(tk, c->hdims, c->ty_sweep);
+  if (c->persistent_km) sort_by_work(tk, c->hdims, c->ty_km);
   // the per-cell kernels (dt, update): 16 planes a tile, fewer where that leaves less than four CTAs per SM
   int kca = 16;
   std::vector<DTile> ta = make_tiles(c->hdims, TY_AUX, kca, 0xe, &c->hkm, -1);
@@ -757,7 +758,8 @@ int mb_init(const mb_mesh* mesh, const mb_scheme* sc, const mb_thermo* th, int d
   c->sc = *sc;
   c->ncell = mesh->ncell_total;
   c->ngroups = ngroups;
-  c->ty_sweep = sc->precision == MB_PREC_MIXED ? TY_F32 : (sc->precision == MB_PREC_FP64_FAST ? TY_F64F : TY_F64);
+  c->ty_sweep = MB_BY_FORM(sc->precision, sweep_unit(sc), _rows, (0));
+  c->ty_km = MB_BY_FORM(sc->precision, sweep_unit(sc), _rows, (1));
   c->no_tma = getenv("MB_NO_TMA") != nullptr;
 #define TRY(x)                 \
   do {                         \
@@ -1631,9 +1633,9 @@ int mb_autotune(mb_ctx* ctx, const double* P, void* stream) {
   ctx->tuned_ms = std::min(ms_plain, ms_pers);
   const std::vector<DTile>& use = ctx->persistent ? sorted : all;
   // the one-plane (mirrored) blocks' list: its own queue mode
-  std::vector<DTile> km = make_tiles(ctx->hdims, ty, ctx->kc3, 0xe, &ctx->hkm, 1);
+  std::vector<DTile> km = make_tiles(ctx->hdims, ctx->ty_km, ctx->kc3, 0xe, &ctx->hkm, 1);
   std::vector<DTile> km_sorted = km;
-  sort_by_work(km_sorted, ctx->hdims, ty);
+  sort_by_work(km_sorted, ctx->hdims, ctx->ty_km);
   float km_plain = 0.f, km_pers = 0.f;
   if (!km.empty()) {
     if ((rc = time_sweep(ctx, km, 0, P, 3, s, &km_plain, 1)) != MB_OK) return rc;

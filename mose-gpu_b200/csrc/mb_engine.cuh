@@ -2082,6 +2082,10 @@ k_sweep(Params p, const DTile* __restrict__ tiles, const double* Pin, const doub
   __shared__ DBlk s_blk;
   __shared__ __align__(8) unsigned long long s_bar;  // TMA staging: the mbarrier of the landing plane
   static_assert(TY <= 8, "one residual slot per warp");
+  // the resident CTAs the registers are capped for have to fit the SM's 228 KB (the arrays above and the 1 KB the system
+  // takes of each CTA are under 2 KB)
+  static_assert(MINB * (sweep_smem<R, TY, VISC, STG, KM, Fast<R>::on && RS != 0>() + 2048) <= 228 * 1024,
+                "registers capped for more CTAs per SM than the tile's shared memory lets in");
   pdl_next();
   TmaStage ts{nullptr, &s_bar, 0u};
   if (Stg<R, STG>::tma) {  // the staging buffer after the tile and the flux buffers, 128-byte aligned

@@ -40,6 +40,11 @@ constexpr int TY_F64 = 5;    // tile rows of the FP64 parity sweep: 160 threads 
 constexpr int TY_F64F = 8;   // tile rows of the FP64 production sweep: 256 threads at 128 registers, 16 warps per SM and an
                              // eighth of the j-faces computed twice. A step of 96^3: 4 rows (128 threads, 232 registers,
                              // 8 warps per SM) 1.71 ms, 6 rows (168 registers, 12 warps) 1.27 ms, 8 rows 1.14 ms
+constexpr int TY_F64F_RS0 = 6;  // the same of the run-time solver unit, which exchanges every face through shared memory:
+                             // 8 rows take 115 KB, one CTA per SM. 192 threads at 168 registers, 2 CTAs, 94 KB each. A step
+                             // of 96^3, HLLE: 4 rows 2.52 ms, 6 rows 1.72 ms, 8 rows 2.68 ms; of 576 x 192 x 64 14.4, 10.6
+                             // and 15.3 ms. One-plane tiles (51 KB at 8 rows) stay at 8: 2-D batch, viscous, 4 rows 1.49 ms,
+                             // 6 rows 1.18 ms, 8 rows 1.02 ms
 constexpr int TY_F32 = 8;    // tile rows of the mixed sweep (256 threads)
 constexpr int MINB_F64 = 2;  // resident CTAs per SM the FP64 sweep's registers must allow
 constexpr int MINB_F32 = 3;  // resident CTAs per SM the mixed sweep's registers must allow (80 registers)
@@ -76,6 +81,7 @@ static inline cudaError_t launch_chained(bool chain, void (*kernel)(K...), unsig
                              cudaStream_t s);                                                                    \
   cudaError_t name##_dt(const Params& p, const DTile* tiles, int ntiles, const double* P, int only_group,       \
                         cudaStream_t s);                                                                         \
+  int name##_rows(int km);                                                                                       \
   int name##_occupancy(int visc, int lim);                                                                       \
   int name##_occupancy_dense(int visc, int lim);                                                                 \
   int name##_occupancy_km(int visc, int lim);

@@ -141,3 +141,19 @@ def test_a_one_cell_axis_with_a_condition_on_one_side_only(engine):
         eng.fill_ghosts()
         assert np.array_equal(eng.state(), P)
         eng.close()
+
+
+@pytest.mark.parametrize("precision", [abi.PREC_FP64, abi.PREC_FP64_FAST, abi.PREC_MIXED])
+@pytest.mark.parametrize("n", [(33, 4, 3), (32, 5, 2), (31, 6, 5), (40, 7, 3), (34, 13, 1)])
+def test_run_time_solver_unit_at_its_tile_edges(engine, n, precision, monkeypatch, capfd):
+    """The run-time solver unit cuts tiles of its own height: one row below, at and above it, and the SM holds as many of
+    its CTAs as the registers are capped for (2 in the FP64 forms, 3 in the mixed one)."""
+    from mosegpu import case as cs
+    monkeypatch.setenv("MB_REPORT", "1")
+    case = cs.duct_3d(widths=(n[0],), heights=(n[1],), depths=(n[2],), mach=1.5, amp=0.02, cfl=0.2, riemann=abi.RS_HLLE,
+                      limiter=abi.LIM_MINMOD, bc={2: abi.BC_EXTRAPOLATION, 3: abi.BC_WALL, 4: abi.BC_SYMMETRY,
+                                                  5: abi.BC_EXTRAPOLATION, 6: abi.BC_EXTRAPOLATION})
+    engine(case, precision=precision).close()
+    report = capfd.readouterr().err
+    assert ", %d CTAs per SM (" % (3 if precision == abi.PREC_MIXED else 2) in report, report
+    _steps(engine, case, precision, 3e-6 if precision == abi.PREC_MIXED else 1e-12, exact=precision == abi.PREC_FP64)
