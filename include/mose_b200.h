@@ -446,17 +446,21 @@ int mb_get_group_status(mb_ctx* ctx, int g0, int n, mb_status* out);
 int mb_read_group_status(mb_ctx* ctx, int g0, int n, mb_status* out, void* stream);
 
 /* The sweep's autotuner (no counterpart in the reference): times, on the state P and the current mesh, the
- * k-chunk of the tiles of 3-D blocks (8 / 16 / 32 / 64 planes) and a plain grid (one CTA per tile) against the
- * persistent work queue (one wave of CTAs taking the largest tiles first from a counter), in the mixed form the
- * staging and 3 or 4 CTAs per SM for 3-D tiles, and keeps the fastest for every later sweep. Does not change P or the clocks; call between steps. */
+ * k-chunk of the tiles of 3-D blocks (8 / 16 / 32 / 64 planes, and the one the engine picks for the mesh by itself) and a
+ * plain grid (one CTA per tile) against the persistent work queue (one wave of CTAs taking the largest tiles first from a
+ * counter), in the mixed form the staging and 3 or 4 CTAs per SM for 3-D tiles, and keeps the fastest for every later
+ * sweep; where the engine's own k-chunk was the fastest, later meshes get theirs. Does not change P or the clocks; call
+ * between steps. */
 int mb_autotune(mb_ctx* ctx, const double* P, void* stream);
 
 /* Sets the sweep configuration by hand: the k-chunk of 3-D tiles and the persistent work queue (1) or the plain
  * grid (0). Synchronises; invalidates the captured step graph. */
 int mb_set_tuning(mb_ctx* ctx, int kchunk, int persistent);
 
-/* The configuration chosen by mb_autotune and its sweep time. Before any call it reports k-chunk 16 and the plain
- * grid; the tiles then take the chunk that fills the device for the mesh (16 where the mesh has no 3-D block). */
+/* The sweep configuration: k-chunk (of the depth class with the most cells), queue mode and, after mb_autotune, the sweep's
+ * time. Before any call the k-chunk is the one that fills the device for the mesh (16 where the mesh has no 3-D block) and
+ * the grid plain. After mb_autotune it is the best of the fixed ones (8 / 16 / 32 / 64), also where the engine's own was
+ * faster and stays in use (MB_REPORT prints the chunks in use). */
 int mb_get_tuning(const mb_ctx* ctx, int* kchunk, int* persistent, float* ms);
 
 /* The tile staging of the mixed form's sweep (no counterpart in the reference): tma = 1 (the default) stages each

@@ -48,11 +48,11 @@ struct mb_ctx {
   int ntiles_km = 0;
   std::vector<int> hkm;         // mirrored-block flag per block
   std::vector<int> hdims;       // 3 per block of the current mesh (interior extents)
-  int kc3 = 16;                 // k-chunk of the sweep tiles of blocks deeper than one cell (mb_set_tuning; the value
-                                // reported by mb_get_tuning: the chunk of the class with the most cells)
+  int kc3 = 16;                 // the k-chunk mb_get_tuning reports (of the class with the most cells): the one in use, after
+                                // mb_autotune the best of its fixed ones
   int kcls[4] = {16, 16, 16, 16};  // the k-chunk per depth class of 3-D blocks (kclass_of): chunk_rule's for the mesh
-                                // until mb_autotune or mb_set_tuning fixes them (tuned)
-  bool tuned = false;
+                                // until mb_autotune (where a fixed chunk is faster) or mb_set_tuning fixes it (tuned)
+  bool tuned[4] = {false, false, false, false};
   int persistent = 0;           // persistent work-queue sweep of the main tile list (autotuned)
   int persistent_km = 0;        // the same for the tiles of mirrored one-plane blocks (autotuned)
   float tuned_ms = 0.f;         // sweep time of the chosen configuration
@@ -186,6 +186,26 @@ static int chunk_rule(const std::vector<int>& dims, int ty, const std::vector<in
     if (c < cost) { cost = c; best = kc; }
   }
   return best;
+}
+
+// the cells and the deepest block (cmaxk, may be null) of each depth class of 3-D blocks; the class with the most cells, -1
+// without any
+static int class_cells(const std::vector<int>& dims, const std::vector<int>& km, long long* ccells, int* cmaxk) {
+  for (int c = 0; c < 4; ++c) {
+    ccells[c] = 0;
+    if (cmaxk) cmaxk[c] = 0;
+  }
+  for (size_t b = 0; b < dims.size() / 3; ++b) {
+    const int* n = &dims[3 * b];
+    if (n[2] <= 1 || km[b] < 0) continue;
+    const int c = kclass_of(n[2]);
+    ccells[c] += (long long)n[0] * n[1] * n[2];
+    if (cmaxk) cmaxk[c] = std::max(cmaxk[c], n[2]);
+  }
+  int big = -1;
+  for (int c = 0; c < 4; ++c)
+    if (ccells[c] && (big < 0 || ccells[c] > ccells[big])) big = c;
+  return big;
 }
 
 // the tile order of a persistent sweep: the largest tiles first, so that the queue ends on small ones
@@ -519,10 +539,12 @@ static int build_tables(mb_ctx* c, const mb_mesh* mesh) {
     for (int a = 0; a < 3; ++a) c->hdims[3 * b + a] = mesh->blk[b].n[a];
   c->hkm.assign(mesh->nblk, 0);
   for (int b = 0; b < mesh->nblk; ++b) c->hkm[b] = mesh->blk[b].group < 0 ? -1 : hb[b].kmirror;
-  if (!c->tuned) {
-    const int kc = chunk_rule(c->hdims, c->ty_sweep, c->hkm, c->p.pgrid);
-    for (int q = 0; q < 4; ++q) c->kcls[q] = kc;
-  }
+  const int kc = chunk_rule(c->hdims, c->ty_sweep, c->hkm, c->p.pgrid);
+  for (int q = 0; q < 4; ++q)
+    if (!c->tuned[q]) c->kcls[q] = kc;
+  long long ccells[4];
+  const int big = class_cells(c->hdims, c->hkm, ccells, nullptr);
+  if (big >= 0) c->kc3 = c->kcls[big];
   std::vector<DTile> ts = make_tiles(c->hdims, c->ty_sweep, c->kc3, 0xe, &c->hkm, 0, c->kcls);
   std::vector<DTile> tk = make_tiles(c->hdims, c->ty_km, c->kc3, 0xe, &c->hkm, 1);
   if (c->persistent) sort_by_work(ts, c->hdims, c->ty_sweep);
@@ -1580,7 +1602,9 @@ int mb_get_status(mb_ctx* ctx, mb_status* st) { return mb_get_group_status(ctx, 
 // The sweep's project-written autotuner, timed on the caller's state over the current mesh (call between steps: it
 // uses the stage buffer):
 //  - per depth class of the 3-D blocks (n3 <= 16, <= 64, <= 256, more; kclass_of), the k-chunk of their tiles
-//    (8, 16, 32 or 64 planes), each class timed over its own tiles;
+//    (8, 16, 32 or 64 planes, or chunk_rule's, which the engine runs untuned), each class timed over its own tiles. One
+//    B200, a step untuned, and tuned without and with the rule's chunk: 53^3 mixed 131, 360 and 129 us, the duct of
+//    121x67x45 312, 406 and 311 us;
 //  - for the main tile list and, separately, for the tiles of the mirrored one-plane blocks (2-D meshes): a plain
 //    grid of one CTA per tile against the persistent work queue (about one wave of CTAs taking tiles, largest first,
 //    from a counter);
@@ -1595,32 +1619,28 @@ int mb_autotune(mb_ctx* ctx, const double* P, void* stream) {
   const int ty = ctx->ty_sweep;
   ctx->dense = false;
   int rc;
-  long long ccells[4] = {0, 0, 0, 0};
-  int cmaxk[4] = {0, 0, 0, 0};
-  for (size_t b = 0; b < ctx->hdims.size() / 3; ++b) {
-    const int* n = &ctx->hdims[3 * b];
-    if (n[2] <= 1 || ctx->hkm[b] < 0) continue;
-    const int c = kclass_of(n[2]);
-    ccells[c] += (long long)n[0] * n[1] * n[2];
-    cmaxk[c] = std::max(cmaxk[c], n[2]);
-  }
-  int big = -1;
+  long long ccells[4];
+  int cmaxk[4];
+  const int big = class_cells(ctx->hdims, ctx->hkm, ccells, cmaxk);
+  const int rule = chunk_rule(ctx->hdims, ty, ctx->hkm, ctx->p.pgrid);
   for (int c = 0; c < 4; ++c) {
     if (!ccells[c]) continue;
-    float best = 1e30f;
-    int kbest = ctx->kcls[c];
+    float best = 1e30f, ms = 0.f;
+    int kbest = 16;
     for (int kc : {8, 16, 32, 64}) {
       if (kc > 16 && kc / 2 >= cmaxk[c]) break;
       std::vector<DTile> tl = make_tiles(ctx->hdims, ty, kc, 1 << 3, &ctx->hkm, 0, nullptr, c);
-      float ms = 0.f;
       if ((rc = time_sweep(ctx, tl, 0, P, 3, s, &ms)) != MB_OK) return rc;
       if (ms < best) { best = ms; kbest = kc; }
     }
-    ctx->kcls[c] = kbest;
-    if (big < 0 || ccells[c] > ccells[big]) big = c;
+    if (c == big) ctx->kc3 = kbest;
+    // the chunk the class runs untuned: where it is faster than all of these, the class keeps it and goes on following
+    // the mesh
+    std::vector<DTile> tl = make_tiles(ctx->hdims, ty, rule, 1 << 3, &ctx->hkm, 0, nullptr, c);
+    if ((rc = time_sweep(ctx, tl, 0, P, 3, s, &ms)) != MB_OK) return rc;
+    ctx->tuned[c] = !(ms < best);
+    ctx->kcls[c] = ctx->tuned[c] ? kbest : rule;
   }
-  ctx->tuned = true;
-  if (big >= 0) ctx->kc3 = ctx->kcls[big];
   std::vector<DTile> all = make_tiles(ctx->hdims, ty, ctx->kc3, 0xe, &ctx->hkm, 0, ctx->kcls);
   std::vector<DTile> sorted = all;
   sort_by_work(sorted, ctx->hdims, ty);
@@ -1715,9 +1735,11 @@ int mb_set_tuning(mb_ctx* ctx, int kchunk, int persistent) {
   CK(cudaSetDevice(ctx->device));
   CK(cudaDeviceSynchronize());
   ctx->kc3 = kchunk;
-  ctx->tuned = true;
   ctx->dense = false;
-  for (int c = 0; c < 4; ++c) ctx->kcls[c] = kchunk;
+  for (int c = 0; c < 4; ++c) {
+    ctx->kcls[c] = kchunk;
+    ctx->tuned[c] = true;
+  }
   ctx->persistent = persistent;
   std::vector<DTile> use = make_tiles(ctx->hdims, ctx->ty_sweep, kchunk, 0xe, &ctx->hkm, 0);
   if (persistent) sort_by_work(use, ctx->hdims, ctx->ty_sweep);
