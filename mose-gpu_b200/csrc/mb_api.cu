@@ -217,11 +217,20 @@ static void sort_by_work(std::vector<DTile>& t, const std::vector<int>& dims, in
   std::stable_sort(t.begin(), t.end(), [&](const DTile& a, const DTile& b) { return w(a) > w(b); });
 }
 
-// The launches of a stage are chained (launch_chained) on meshes of at most one tile per SM. On more, the CTAs that a
-// kernel places while the one before still runs go where slots happen to be free, and the uneven placement costs more
-// than the gaps: one B200, a step of 1-D, 1000 cells (32 tiles) 68 us unchained and 60 us chained, but 53^3 mixed (378
-// tiles) 160 and 199 us, 2-D 301^2 (380 tiles) 86 and 88 us.
-static void set_chain(mb_ctx* c) { c->p.chain = c->ntiles_sweep + c->ntiles_km <= c->nsm; }
+// The launches of a stage are chained (launch_chained) on the smallest meshes: tiles of one plane, at most one per SM (of
+// 3-D blocks one per two SMs). The CTAs that a kernel places while the one before still runs go where slots happen to be
+// free, several to an SM, and the uneven placement costs more than the gaps where there are more tiles or longer ones.
+// One B200, a step unchained and chained: 1-D, 1000 cells (32 tiles) 53.6 and 45.4 us, 2-D 128^2 (64) 61.5 and 55.2, 180^2
+// (138) 60.5 and 55.6, 3-D 24^3 (72 tiles of a plane) 84.2 and 78.2; but 32 x 24 x 40 (120) 83.8 and 86.4, 53^3 in 378
+// tiles of two planes 160 and 199, in 98 of eight 256 and 368, 64^3 in 64 of sixteen 765 and 1124.
+static void set_chain(mb_ctx* c, const std::vector<DTile>& main) {
+  int n3 = 0, planes = 1;
+  for (const DTile& t : main) {
+    planes = std::max(planes, t.k1 - t.k0);
+    n3 += c->hdims[3 * t.blk + 2] > 1;
+  }
+  c->p.chain = planes == 1 && 2 * n3 <= c->nsm && (int)main.size() + c->ntiles_km <= c->nsm;
+}
 
 static const double RKC[3][3] = {{1.0, 0.0, 0.0}, {1.0, 0.50, 0.0}, {1.0, 0.25, 2.0 / 3.0}};  // Lib_RK.f90:6-9
 
@@ -679,7 +688,7 @@ static int build_tables(mb_ctx* c, const mb_mesh* mesh) {
     return MB_E_NOMEM;
   c->ntiles_sweep = (int)ts.size();
   c->ntiles_aux = (int)ta.size();
-  set_chain(c);
+  set_chain(c, ts);
   Params& p = c->p;
   p.blk = c->d_blk; p.rec_map = c->d_recmap; p.rec = c->d_rec; p.pgsrc = c->d_pgsrc;
   p.recflux = c->d_recflux;
@@ -1707,7 +1716,7 @@ int mb_autotune(mb_ctx* ctx, const double* P, void* stream) {
   if ((rc = upload(&ctx->d_tiles_km, use_km.data(), use_km.size())) != MB_OK) return rc;
   ctx->ntiles_sweep = (int)use.size();
   ctx->ntiles_km = (int)use_km.size();
-  set_chain(ctx);
+  set_chain(ctx, use);
   CK(cudaStreamSynchronize(0));
   if (ctx->gexec) { cudaGraphExecDestroy(ctx->gexec); ctx->gexec = nullptr; }
   if (ctx->graph) { cudaGraphDestroy(ctx->graph); ctx->graph = nullptr; }
@@ -1748,7 +1757,7 @@ int mb_set_tuning(mb_ctx* ctx, int kchunk, int persistent) {
   int rc = upload(&ctx->d_tiles_sweep, use.data(), use.size());
   if (rc != MB_OK) return rc;
   ctx->ntiles_sweep = (int)use.size();
-  set_chain(ctx);
+  set_chain(ctx, use);
   if (ctx->gexec) { cudaGraphExecDestroy(ctx->gexec); ctx->gexec = nullptr; }
   if (ctx->graph) { cudaGraphDestroy(ctx->graph); ctx->graph = nullptr; }
   ctx->gP = nullptr;

@@ -106,3 +106,19 @@ def test_depth_classes_nobody_timed_follow_the_mesh():
     one = Engine(cs.riemann_1d(n=64))
     assert one.tuning()[:2] == (16, 0)
     one.close()
+
+
+def test_a_step_of_few_long_tiles_takes_no_longer_than_its_parts():
+    """64^3 in 64 tiles of 16 planes, fewer than the SMs: a step's launches one after another take what its ghost fills and
+    sweeps take by themselves. Chained, their tiles shared SMs and the step took 1.37 times that."""
+    torch = pytest.importorskip("torch")
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from mosegpu import case as cs
+    from mosegpu.engine import Engine
+    eng = Engine(cs.taylor_green(n=64), precision=abi.PREC_MIXED)
+    eng.set_tuning(16, False)
+    step = _step_us(torch, eng)
+    parts = sum(sum(eng.profile_stage(q, 20)) for q in (1, 2, 3)) * 1e3
+    assert step <= 1.15 * parts, (step, parts)
+    eng.close()
