@@ -71,6 +71,7 @@ struct mb_ctx {
   bool stage_tma = true;        // the mixed sweep stages by TMA where a map exists (mb_set_staging, mb_autotune)
   bool stage_tma_km = true;     // the same for the tile list of mirrored one-plane blocks (tuned separately)
   bool dense = false;           // Params::dense of the main tile list (mb_autotune, with plain staging)
+  bool stage_tma_alt = true;    // stage_tma without it
   cudaStream_t tstream = 0;     // the stream the mesh tables are (re)built in the order of (build_tables)
   long long sweeps_tma = 0, sweeps_plain = 0;  // sweep launches of the mixed form by staging path
   double* d_acc4 = nullptr;     // RK4: conserved accumulator (ncell x 5)
@@ -233,6 +234,13 @@ static void set_chain(mb_ctx* c, const std::vector<DTile>& main) {
 }
 
 static const double RKC[3][3] = {{1.0, 0.0, 0.0}, {1.0, 0.50, 0.0}, {1.0, 0.25, 2.0 / 3.0}};  // Lib_RK.f90:6-9
+
+// back from the dense form to the staging measured without it
+static void leave_dense(mb_ctx* c) {
+  if (!c->dense) return;
+  c->dense = false;
+  c->stage_tma = c->stage_tma_alt;
+}
 
 // rk_coeff of stage irk (the SSP forms); RK4 carries its own weights in the update (cons_update)
 static double rkc_of(int n, int irk) { return n == 4 ? 0.0 : RKC[n - 1][irk - 1]; }
@@ -1626,7 +1634,7 @@ int mb_autotune(mb_ctx* ctx, const double* P, void* stream) {
   cudaStream_t s = (cudaStream_t)stream;
   prepare_tmaps(ctx, P, P, s);
   const int ty = ctx->ty_sweep;
-  ctx->dense = false;
+  leave_dense(ctx);
   int rc;
   long long ccells[4];
   int cmaxk[4];
@@ -1695,14 +1703,14 @@ int mb_autotune(mb_ctx* ctx, const double* P, void* stream) {
     // the 3-D sweep at 4 CTAs per SM instead of 3: a third more warps to cover latency, but 64 registers and an L1 of
     // 28 KB instead of 92. It wins where the geometry stays in the caches (one B200, 64 blocks of 32^3 that share it, a
     // step 1215 and 1068 us) and loses where it streams (192^3 in one block 2.82 and 3.03 ms), so it is timed
-    if (!use.empty() && ctx->p.pgrid_dense > ctx->p.pgrid) {
-      const bool tma = ctx->stage_tma;
+    // (residual smoothing runs the residual sweep, which has no such form)
+    if (!use.empty() && ctx->sc.irs <= 0 && ctx->p.pgrid_dense > ctx->p.pgrid) {
       float ms = 0.f;
+      ctx->stage_tma_alt = ctx->stage_tma;
       ctx->stage_tma = false;
       ctx->dense = true;
       rc = time_sweep(ctx, use, ctx->persistent, P, 3, s, &ms);
-      ctx->dense = rc == MB_OK && ms < best;
-      if (!ctx->dense) ctx->stage_tma = tma;
+      if (rc != MB_OK || !(ms < best)) leave_dense(ctx);
       if (rc != MB_OK) return rc;
       best = std::min(best, ms);
     }
@@ -1744,7 +1752,7 @@ int mb_set_tuning(mb_ctx* ctx, int kchunk, int persistent) {
   CK(cudaSetDevice(ctx->device));
   CK(cudaDeviceSynchronize());
   ctx->kc3 = kchunk;
-  ctx->dense = false;
+  leave_dense(ctx);
   for (int c = 0; c < 4; ++c) {
     ctx->kcls[c] = kchunk;
     ctx->tuned[c] = true;

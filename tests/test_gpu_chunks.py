@@ -122,3 +122,27 @@ def test_a_step_of_few_long_tiles_takes_no_longer_than_its_parts():
     parts = sum(sum(eng.profile_stage(q, 20)) for q in (1, 2, 3)) * 1e3
     assert step <= 1.15 * parts, (step, parts)
     eng.close()
+
+
+@pytest.mark.parametrize("irs", [0, 2])
+def test_the_staging_is_the_one_measured_for_the_sweeps_that_run(irs, monkeypatch, capfd):
+    """The 4-CTA form of the 3-D sweep stages by plain loads. Where it does not run, with residual smoothing (whose sweeps
+    write residuals) or after mb_set_tuning, the staging is the faster of the two timed without it."""
+    import re
+    torch = pytest.importorskip("torch")
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from mosegpu import case as cs
+    from mosegpu.engine import Engine
+    case = cs.taylor_green(n=128, blocks=4, riemann=abi.RS_HLLC, share_geometry=True)
+    case.scheme["irs"] = irs
+    eng = Engine(case, precision=abi.PREC_MIXED)
+    eng.fill_ghosts()
+    monkeypatch.setenv("MB_REPORT", "1")
+    eng.autotune()
+    six, five = re.search(r"main list:.*?\(6-value ([\d.]+) ms, 5-value ([\d.]+) ms\)", capfd.readouterr().err).groups()
+    if not irs:
+        eng.set_tuning(8, False)
+    if six != five:
+        assert eng.staging_mode() == (float(five) < float(six)), (six, five)
+    eng.close()
