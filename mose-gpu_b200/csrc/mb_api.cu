@@ -556,7 +556,7 @@ static int build_tables(mb_ctx* c, const mb_mesh* mesh) {
     for (int a = 0; a < 3; ++a) c->hdims[3 * b + a] = mesh->blk[b].n[a];
   c->hkm.assign(mesh->nblk, 0);
   for (int b = 0; b < mesh->nblk; ++b) c->hkm[b] = mesh->blk[b].group < 0 ? -1 : hb[b].kmirror;
-  const int kc = chunk_rule(c->hdims, c->ty_sweep, c->hkm, c->p.pgrid);
+  const int kc = chunk_rule(c->hdims, c->ty_sweep, c->hkm, c->dense ? c->p.pgrid_dense : c->p.pgrid);
   for (int q = 0; q < 4; ++q)
     if (!c->tuned[q]) c->kcls[q] = kc;
   long long ccells[4];
@@ -1640,10 +1640,11 @@ int mb_autotune(mb_ctx* ctx, const double* P, void* stream) {
   int cmaxk[4];
   const int big = class_cells(ctx->hdims, ctx->hkm, ccells, cmaxk);
   const int rule = chunk_rule(ctx->hdims, ty, ctx->hkm, ctx->p.pgrid);
+  int kfix[4] = {16, 16, 16, 16};  // the best of the fixed chunks per class
   for (int c = 0; c < 4; ++c) {
     if (!ccells[c]) continue;
     float best = 1e30f, ms = 0.f;
-    int kbest = 16;
+    int& kbest = kfix[c];
     for (int kc : {8, 16, 32, 64}) {
       if (kc > 16 && kc / 2 >= cmaxk[c]) break;
       std::vector<DTile> tl = make_tiles(ctx->hdims, ty, kc, 1 << 3, &ctx->hkm, 0, nullptr, c);
@@ -1668,7 +1669,7 @@ int mb_autotune(mb_ctx* ctx, const double* P, void* stream) {
   }
   ctx->persistent = ms_pers < ms_plain ? 1 : 0;
   ctx->tuned_ms = std::min(ms_plain, ms_pers);
-  const std::vector<DTile>& use = ctx->persistent ? sorted : all;
+  std::vector<DTile> use = ctx->persistent ? sorted : all;
   // the one-plane (mirrored) blocks' list: its own queue mode
   std::vector<DTile> km = make_tiles(ctx->hdims, ctx->ty_km, ctx->kc3, 0xe, &ctx->hkm, 1);
   std::vector<DTile> km_sorted = km;
@@ -1703,16 +1704,36 @@ int mb_autotune(mb_ctx* ctx, const double* P, void* stream) {
     // the 3-D sweep at 4 CTAs per SM instead of 3: a third more warps to cover latency, but 64 registers and an L1 of
     // 28 KB instead of 92. It wins where the geometry stays in the caches (one B200, 64 blocks of 32^3 that share it, a
     // step 1215 and 1068 us) and loses where it streams (192^3 in one block 2.82 and 3.03 ms), so it is timed
-    // (residual smoothing runs the residual sweep, which has no such form)
+    // (residual smoothing runs the residual sweep, which has no such form). A third more slots want other chunks and
+    // another queue mode: the best fixed chunks and the rule's for those slots, both ways. The 64 blocks, a step with the
+    // chunk of the 3-CTA form only 1124 us, with these 1080 us.
     if (!use.empty() && ctx->sc.irs <= 0 && ctx->p.pgrid_dense > ctx->p.pgrid) {
-      float ms = 0.f;
+      const int rd = chunk_rule(ctx->hdims, ty, ctx->hkm, ctx->p.pgrid_dense);
+      const int krule[4] = {rd, rd, rd, rd};
+      int pers = ctx->persistent;
+      bool won = false, fixed = false;
       ctx->stage_tma_alt = ctx->stage_tma;
       ctx->stage_tma = false;
       ctx->dense = true;
-      rc = time_sweep(ctx, use, ctx->persistent, P, 3, s, &ms);
-      if (rc != MB_OK || !(ms < best)) leave_dense(ctx);
-      if (rc != MB_OK) return rc;
-      best = std::min(best, ms);
+      for (int m = 0; m < 4; ++m) {
+        const int* kc = m < 2 ? kfix : krule;
+        std::vector<DTile> tl = make_tiles(ctx->hdims, ty, ctx->kc3, 0xe, &ctx->hkm, 0, kc);
+        if (m & 1) sort_by_work(tl, ctx->hdims, ty);
+        float ms = 0.f;
+        rc = time_sweep(ctx, tl, m & 1, P, 3, s, &ms);
+        if (rc != MB_OK) { leave_dense(ctx); return rc; }
+        if (ms < best) { best = ms; won = true; fixed = m < 2; pers = m & 1; use = tl; }
+      }
+      if (won) {
+        ctx->persistent = pers;
+        for (int c = 0; c < 4; ++c) {
+          if (!ccells[c]) continue;
+          ctx->kcls[c] = fixed ? kfix[c] : rd;
+          ctx->tuned[c] = fixed;
+        }
+      } else {
+        leave_dense(ctx);
+      }
     }
     ctx->tuned_ms = best + std::min(ms_stage_km[0], ms_stage_km[1]);
   }
