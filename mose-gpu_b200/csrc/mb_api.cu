@@ -34,7 +34,7 @@ struct mb_ctx {
   long long* d_cdst = nullptr;
   long long* d_csrc = nullptr;
   long long* d_pgsrc = nullptr;
-  double* d_recflux = nullptr;  // boundary-record contributions [nrec][10] (flux type)
+  double* d_recflux = nullptr;  // boundary-record contributions (Params::recflux)
   RecWork* d_work = nullptr;    // records in type order (the record kernel's work list)
   int nrec = 0;
   double* d_tab = nullptr;

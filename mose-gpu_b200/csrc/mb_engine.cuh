@@ -1068,11 +1068,13 @@ __device__ __forceinline__ void clock_groups(const Params& p) {
 
 // Every boundary record of the mesh, one thread each, from the stage input P (ghosts filled): the contributions
 // (A, S) of record q go to recflux[q][0..9] in the flux type, or, on the simplified flux path of the solvers with their
-// own unit, the net one (A - S) to recflux[q][0..4]; the sweep adds them in face order after the interior sum
-// (BC_Fluxes after Fluxes, Mod_Explicit.f90:187-189). A warp's time is its chain of dependent loads, so what a record
-// needs to find its cells is one 32-byte entry (RecWork), and the connection records of that path take the interior
-// face's code and the FP32 geometry: one B200, a step with the records before and with them, 64 blocks of 32^3 mixed
-// 1572 and 1451 us, duct 121x67x45 430 and 399 us, 53^3 202 and 191 us.
+// own unit, A - S to recflux[q][0..4] in FP64 (in FP32 the difference would round S to the ulp of A, the pressure on a
+// wall); the sweep adds them in FP64 in face order after the interior sum (BC_Fluxes after Fluxes,
+// Mod_Explicit.f90:187-189). A warp's time is its chain of dependent loads, so what a record needs to find its cells is
+// one 32-byte entry (RecWork), and the connection records of that path take the interior face's code and the FP32
+// geometry: one B200, a step with the records before and with them, 64 blocks of 32^3 mixed 1572 and 1451 us, duct
+// 121x67x45 430 and 399 us, 53^3 202 and 191 us. Against A and S as 10 FP32 values: the 64 blocks 1095 and 1115 us,
+// the duct 322 and 328, the 2-D batch of 12 blocks 540 and 555.
 // VAR tells apart the instantiations of the same types built with different flags (the FP64 production form's units)
 template <typename R, bool VISC, int RS, int LIM, int VAR = 0>
 __global__ void __launch_bounds__(128) k_records(Params p, const RecWork* __restrict__ work, int nrec,
@@ -1099,23 +1101,16 @@ __global__ void __launch_bounds__(128) k_records(Params p, const RecWork* __rest
   // Where the clock shares the launch it may be setting the flag now, so its records are computed whatever the flag says
   // (those of a case that has just ended are not read: its tiles return).
   if (!sf.clock && p.st[b.grp].done) return;
+  R v[2 * MB_NP];
   if constexpr (Fast<R>::on && RS != 0) {
-    R v[MB_NP];
-    if (type == 1) {
-      conn_fast<R, VISC, RS, LIM>(p, b, P, w0.y, w0.z, w0.w, face, p.pgsrc + (long long)w1.w * 6, v);
-    } else {
-      R S[MB_NP];
-      bc_record<R, VISC, RS, LIM>(p, b, P, rid, w0.y, w0.z, w0.w, face, v, S);
-      if (VISC) {
+    if (type == 1)
+      conn_fast<R, VISC, RS, LIM>(p, b, P, w0.y, w0.z, w0.w, face, p.pgsrc + (long long)w1.w * 6, v, v + MB_NP);
+    else
+      bc_record<R, VISC, RS, LIM>(p, b, P, rid, w0.y, w0.z, w0.w, face, v, v + MB_NP);
+    double* out = static_cast<double*>(p.recflux) + (long long)rid * MB_NP;
 #pragma unroll
-        for (int s = 0; s < MB_NP; ++s) v[s] = v[s] - S[s];
-      }
-    }
-    R* out = reinterpret_cast<R*>(p.recflux) + (long long)rid * MB_NP;
-#pragma unroll
-    for (int s = 0; s < MB_NP; ++s) out[s] = v[s];
+    for (int s = 0; s < MB_NP; ++s) out[s] = VISC ? (double)v[s] - (double)v[MB_NP + s] : (double)v[s];
   } else {
-    R v[2 * MB_NP];
     bc_record<R, VISC, RS, LIM>(p, b, P, rid, w0.y, w0.z, w0.w, face, v, v + MB_NP);
     R* out = reinterpret_cast<R*>(p.recflux) + (long long)rid * 2 * MB_NP;
 #pragma unroll
@@ -1949,8 +1944,13 @@ __device__ __forceinline__ bool sweep_tile(const Params& p, const DTile t, const
           if (!((on >> (F - 1)) & 1)) continue;
           const int rid = record_of(p, b, F, i, j, k);
           if (rid >= 0) {
-            if constexpr (PAIR) bc_apply<R, false>(rf + (long long)rid * MB_NP, acc);
-            else bc_apply<R, VISC>(rf + (long long)rid * 2 * MB_NP, acc);
+            if constexpr (PAIR) {
+              const double* net = static_cast<const double*>(p.recflux) + (long long)rid * MB_NP;
+#pragma unroll
+              for (int s = 0; s < MB_NP; ++s) acc[s] = acc[s] + net[s];
+            } else {
+              bc_apply<R, VISC>(rf + (long long)rid * 2 * MB_NP, acc);
+            }
           }
         }
         if (KM) {  // faces 5 and 6 of a mirrored block: the extrapolation records of every cell, computed here

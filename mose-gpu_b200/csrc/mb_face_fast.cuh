@@ -256,12 +256,13 @@ __device__ __forceinline__ void ausm_pair(const Params& p, const Side<R>& L, con
 }
 
 // The net flux (convective - viscous) along +d of the face between padded cell l0 of block b and its +d neighbour (gst
-// further on), into out[0..4]. c gives the states: c.stencil(q, A, B, C), q = 0..3, the four cells along d (1 and 2 the
-// face's own); c.transverse(e, w, A, B) the neighbours along the two other axes e in increasing order (w = 0, 1: below /
-// above cell 1; 2, 3: below / above cell 2).
+// further on), into out[0..4]; where vout is given (the records), the convective one into out and the viscous one into
+// vout. c gives the states: c.stencil(q, A, B, C), q = 0..3, the four cells along d (1 and 2 the face's own);
+// c.transverse(e, w, A, B) the neighbours along the two other axes e in increasing order (w = 0, 1: below / above cell 1;
+// 2, 3: below / above cell 2).
 template <typename R, bool VISC, int RS, int LIM, typename Cells>
 __device__ __forceinline__ void face_core(const Params& p, const DBlk& b, int d, int l0, int gst, int face,
-                                          const Cells& c, R* out) {
+                                          const Cells& c, R* out, R* vout = nullptr) {
   R nx, ny, nz, area;
   face_rec(b, d, face, nx, ny, nz, area);
   if (nx == (R)0 && ny == (R)0 && nz == (R)0) area = (R)0;  // a degenerate face carries no flux
@@ -360,7 +361,14 @@ __device__ __forceinline__ void face_core(const Params& p, const DBlk& b, int d,
   if (RS == 12) roe_pair<R>(p, L, Q, nx, ny, nz, fr, fuv, fw, fe);
   else if (RS == 1) hllc_pair<R>(p, L, Q, nx, ny, nz, fr, fuv, fw, fe);
   else ausm_pair<R>(p, L, Q, nx, ny, nz, fr, fuv, fw, fe);
-  if (VISC) {
+  if (VISC && vout) {
+    const V2<R> G = vuv * dup2<R>(area);
+    vout[0] = (R)0;
+    vout[MB_IU] = lo2(G);
+    vout[MB_IV] = hi2(G);
+    vout[MB_IW] = vw * area;
+    vout[MB_IPR] = ve * area;
+  } else if (VISC) {
     fuv = fuv - vuv;
     fw = fw - vw;
     fe = fe - ve;
@@ -432,12 +440,12 @@ struct ArenaCells {
   __device__ __forceinline__ static long long ld_row(const long long* q) { return __ldg(q); }
 };
 
-// a connection record (bc_conn_eul and bc_conn_visc of mb_engine.cuh): the net contribution to the row of its cell. The
-// two viscous fluxes the reference averages, with the gradients of the cell and of its ghost, are one flux with the
+// a connection record (bc_conn_eul and bc_conn_visc of mb_engine.cuh): its contributions A and S to the row of its cell.
+// The two viscous fluxes the reference averages, with the gradients of the cell and of its ghost, are one flux with the
 // mean gradient (the flux is linear in it): the interior face's.
 template <typename R, bool VISC, int RS, int LIM>
 __device__ __forceinline__ void conn_fast(const Params& p, const DBlk& b, const double* P, int i, int j,
-                                          int k, int F, const long long* __restrict__ pg, R* out) {
+                                          int k, int F, const long long* __restrict__ pg, R* A, R* S) {
   const int d = (F - 1) >> 1, low = F & 1;
   const int gst = (d == 0) ? 1 : (d == 1 ? b.pi : b.pi * b.pj);
   const int l = lin32(b, i, j, k);
@@ -445,10 +453,13 @@ __device__ __forceinline__ void conn_fast(const Params& p, const DBlk& b, const 
   const int sk = b.kmirror ? 0 : b.pi * b.pj;  // a mirrored block's k ghosts are its k = 1 cells
   const ArenaCells<R> c{P, p.nc, b.boff + l - low * gst, gst, b.boff + l, (d == 0) ? b.pi : 1, (d == 2) ? b.pi : sk, pg,
                         Cst<R>::of(p).iri, low != 0};
-  face_core<R, VISC, RS, LIM>(p, b, d, l - low * gst, gst, fmi32(b, d, il, jl, kl), c, out);
+  face_core<R, VISC, RS, LIM>(p, b, d, l - low * gst, gst, fmi32(b, d, il, jl, kl), c, A, S);
   if (low) {
 #pragma unroll
-    for (int s = 0; s < MB_NP; ++s) out[s] = -out[s];
+    for (int s = 0; s < MB_NP; ++s) {
+      A[s] = -A[s];
+      if (VISC) S[s] = -S[s];
+    }
   }
 }
 

@@ -156,7 +156,7 @@ struct Params {
   int cfl_rise;            // cfl-rise-threshold (0: no ramp)
   int lim, rs, visc, ndir, dt_additive, guard, state_check;
   double cfl, vnn, prandtl, schmidt, mco;
-  void* recflux;           // boundary-record contributions [record][10] in the flux type (k_records)
+  void* recflux;           // boundary-record contributions (k_records): [record][10] in the flux type, or [record][5] in FP64
   int stg;                 // mixed form: the tile staging of the sweep (STG_PLAIN 0, STG_TMA 1 of mb_engine.cuh)
   const void* tmap;        // STG_TMA: the TMA tensor map (CUtensorMap, device memory) of the sweep's input state as a
                            // 2-D tensor of (ncell_total rows, 5 variables), or null (the same tile by plain loads)

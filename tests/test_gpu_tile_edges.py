@@ -185,3 +185,36 @@ def test_hllc_star_flux_has_no_cancellation(engine):
     for v in (0, 1, 4):
         e = np.sqrt(np.mean((got[v] - ref[v]) ** 2)) / (area * np.sqrt(np.mean(scale[v] ** 2)))
         assert e <= 3e-7, (v, e)
+
+
+def test_wall_friction_below_an_ulp_of_the_pressure_is_kept(engine):
+    """A record's convective and viscous contributions are FP32 values added one after the other in FP64: the friction of an
+    inclined wall shows in the mixed form's residual although it is below an FP32 rounding of the pressure on that wall. A
+    uniform stream along the walls of a rotated channel has no other viscous flux, so the difference of two residuals with
+    different viscosities is the friction's; to 1e-5 (a few FP32 roundings of the friction itself) it is the FP64 form's."""
+    from mosegpu import case as cs
+    co, si, n = np.cos(0.5), np.sin(0.5), (40, 9, 1)
+    R = cs.ideal_gas_tables()["R"]
+    diff = []
+    for precision in (abi.PREC_FP64, abi.PREC_MIXED):
+        res = []
+        for mu in (2.5e-7, 5e-7):
+            def nodes(i, j, k):
+                x, y = i / 40.0, j / 40.0
+                return np.stack([co * x - si * y, si * x + co * y, k / 40.0], axis=-1)
+
+            def prim(c):
+                return np.stack([np.full(c.shape[:-1], v) for v in (1e5 / (R * 300.0), 100.0 * co, 100.0 * si, 0.0, 1e5)])
+            sch = dict(limiter=abi.LIM_MINMOD, riemann=abi.RS_HLLC, visc=1, n_rk=3, ndir=2, cfl=0.4, prandtl=0.71)
+            case = cs.layout_case("rotated", [[0, q] for q in n], nodes, (False,) * 3,
+                                  {1: abi.BC_EXTRAPOLATION, 2: abi.BC_EXTRAPOLATION, 3: abi.BC_WALL, 4: abi.BC_WALL,
+                                   5: abi.BC_EXTRAPOLATION, 6: abi.BC_EXTRAPOLATION}, cs.ideal_gas_tables(mu=mu), sch, prim)
+            eng = engine(case, precision=precision)
+            eng.fill_ghosts()
+            r = case.interior(eng.residual().cpu().numpy(), 0)
+            res.append(np.concatenate([r[1:3, 2:-2, 0], r[1:3, 2:-2, -1]]))
+            eng.close()
+        diff.append(res[1] - res[0])
+    scale = np.abs(diff[0]).max()
+    assert 0 < scale < 1e5 / 40 ** 2 * 6e-8  # below an ulp of the pressure force
+    assert np.abs(diff[1] - diff[0]).max() < 1e-5 * scale, (np.abs(diff[1]).max(), scale)
