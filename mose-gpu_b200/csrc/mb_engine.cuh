@@ -232,7 +232,6 @@ MB_HD void bc_face_geom(const DBlk& b, int Im, int Jm, int Km, int F, double* g)
 template <typename R, int RS = 0, int LIM = 0>
 MB_HD void bc_conn_eul(const Params& p, const DBlk& b, const double* P, int Im, int Jm, int Km, int Fm, R* A) {
   const long long nc = p.nc;
-  const int rs = RS ? RS : p.rs;
   const int lim = LIM ? LIM : p.lim;
   int dir = (Fm + 1) / 2, modfm = Fm % 2, modfm1 = 1 - modfm, modfm2 = 1 - 2 * modfm, gstep = 2 * modfm - 1;
   int o[4] = {modfm * (-gstep * GC) + modfm1 * gstep, modfm * (-gstep), modfm1 * (-gstep),
@@ -945,14 +944,14 @@ MB_HD int record_of(const Params& p, const DBlk& b, int F, int i, int j, int k) 
 
 // One boundary record (bc_record_apply.inc): its contributions to the cell's R row, in the flux type. A is added
 // and then, in Navier-Stokes, S is subtracted (the order of the reference's statements); components a record leaves
-// alone hold exact no-ops (-0 in A, +0 in S).
-template <typename R, bool VISC, int RS = 0, int LIM = 0>
+// alone hold exact no-ops (-0 in A, +0 in S). CONN = false: connection records go elsewhere (conn_fast).
+template <typename R, bool VISC, int RS = 0, int LIM = 0, bool CONN = true>
 MB_HD void bc_record(const Params& p, const DBlk& b, const double* P, int rid, int i, int j, int k, int F,
                      R* A, R* S) {
   const DRec& rc = p.rec[rid];
   if (VISC)
     for (int s = 0; s < MB_NP; ++s) S[s] = (R)0;
-  if (rc.type == 1) {
+  if (CONN && rc.type == 1) {
     bc_conn_eul<R, RS, LIM>(p, b, P, i, j, k, F, A);
     if (VISC) bc_conn_visc<R>(p, b, P, i, j, k, F, p.pgsrc + (long long)rc.pg * 6, S);
   } else if (rc.type == 11) {
@@ -1106,7 +1105,7 @@ __global__ void __launch_bounds__(128) k_records(Params p, const RecWork* __rest
     if (type == 1)
       conn_fast<R, VISC, RS, LIM>(p, b, P, w0.y, w0.z, w0.w, face, p.pgsrc + (long long)w1.w * 6, v, v + MB_NP);
     else
-      bc_record<R, VISC, RS, LIM>(p, b, P, rid, w0.y, w0.z, w0.w, face, v, v + MB_NP);
+      bc_record<R, VISC, RS, LIM, false>(p, b, P, rid, w0.y, w0.z, w0.w, face, v, v + MB_NP);
     double* out = static_cast<double*>(p.recflux) + (long long)rid * MB_NP;
 #pragma unroll
     for (int s = 0; s < MB_NP; ++s) out[s] = VISC ? (double)v[s] - (double)v[MB_NP + s] : (double)v[s];
