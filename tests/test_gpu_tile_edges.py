@@ -1,6 +1,7 @@
-"""The simplified flux path (paired values, faces summed in registers, shuffles and shared exchange rows) and the merged
-surface launches at the sizes where they can go wrong: one cell below, at and above the 32 x 8 tiles, axes of one to three
-cells, every limiter, the three solvers with their own unit, walls, inlet, outflow, symmetry and connections.
+"""The simplified flux path (paired values, faces summed in registers, shuffles and shared exchange rows) and the one-launch
+ghost fill at the sizes where they can go wrong: one cell below, at and above the 32 x 8 tiles, axes of one to three cells,
+every limiter, the three solvers with their own unit, walls, inlet, outflow, symmetry and connections. (The launch that
+also carries the records and the clock is in test_gpu_surface.py.)
 
 Tolerances: the FP64 production form against the oracle at the north-star gate of one step (1e-12, max-norm relative to
 the field, momentum against its vector); the parity form bit for bit. The mixed form: every face flux carries a few FP32
@@ -85,8 +86,9 @@ BCS = {"wall": abi.BC_WALL, "extrapolation": abi.BC_EXTRAPOLATION, "symmetry": a
 @pytest.mark.parametrize("low,high", [("wall", "wall"), ("wall", "extrapolation"), ("symmetry", "extrapolation"),
                                       ("extrapolation", "extrapolation"), ("symmetry", "none")])
 def test_thin_axes_take_the_general_fill(engine, low, high, n2, visc):
-    """The rules that merge the ghost passes, and the records with them, against the sequential fill of the oracle: every
-    pair of face types on an axis of one, two and three cells, bit for bit."""
+    """The rules that merge the ghost passes, on a mesh with connections, against the sequential fill of the oracle: every
+    pair of face types on an axis of one, two and three cells, bit for bit. (Viscous walls one or two cells apart are left
+    out: their ghosts start from ghosts that are zero here, and the oracle's field leaves the tables.)"""
     from mosegpu import case as cs
     case = cs.multiblock_2d(cols=2, rows=1, widths=[6, 35], heights=[n2], visc=visc, mach=0.5, n_rk=3, cfl=0.2,
                             riemann=abi.RS_HLLC, limiter=abi.LIM_MINMOD,
