@@ -1798,8 +1798,7 @@ __device__ __forceinline__ bool sweep_tile(const Params& p, const DTile t, const
     __syncthreads();  // plane k+2 staged, and every pass 2 of plane k-1 done (the flux buffers are free)
     // the next plane's boxes fly under this plane's faces and pass 2 (the staging buffer was read before the barrier)
     if (tma && k + 3 <= b.n3 + kext && k + 1 < t.k1) tma_issue_plane<TY>(p, b, raw, bar, t.i0, t.j0, k + 3);
-    // ---- face tasks of this plane through one call site: 0 = i-face #tid, 1 = extra i-faces (last warp,
-    // lanes < TY), 2 = j-face #tid, 3 = extra j-face row (warp 0), 4 = the k-face above
+    // ---- the faces of this plane
     R net[NS];
     if constexpr (PAIR) {
       // one call site per direction: with a literal d the offsets and pointers need no selects, and the shorter face code
@@ -1854,6 +1853,8 @@ __device__ __forceinline__ bool sweep_tile(const Params& p, const DTile t, const
         }
       }
     } else {
+    // face tasks through one call site: 0 = i-face #tid, 1 = extra i-faces (last warp, lanes < TY), 2 = j-face #tid,
+    // 3 = extra j-face row (warp 0), 4 = the k-face above
 #pragma unroll 1
     for (int task = 0; task < 5; ++task) {
       int d = -1, fi = 0, fj = 0, ii = 0, jj = 0;

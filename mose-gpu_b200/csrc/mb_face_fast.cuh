@@ -1,7 +1,8 @@
 // mb_face_fast.cuh -- the interior face flux of the simplified flux path (the mixed form and the FP64 production form)
 // for the solvers with their own sweep unit: HLLC (1), AUSM+ (4), LMRoe (12). The same scheme as face_flux of
 // mb_engine.cuh (conv_physics.inc, diff_cuf_kernels.inc, diff_physics.inc) with the single-species identities, written
-// for few instructions, which is what bounds the sweep (its DRAM traffic is under a fifth of the peak):
+// for few instructions, which bounded the sweep before it (60 % of the issue slots in use, DRAM under a fifth of its peak;
+// with it half of the slots are, and exposed latency bounds it):
 //  - values travel in pairs, (u, v), (w, T), (rho, p): one 8-byte shared load brings two, and in FP32 one instruction
 //    (add / mul / fma .f32x2, each half rounded as the scalar instruction rounds) computes on both;
 //  - a divide is a multiplication by a reciprocal; in FP32 the reciprocal is one instruction (rcp.approx.ftz), where

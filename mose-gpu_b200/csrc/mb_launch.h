@@ -1,6 +1,6 @@
-// mb_launch.h -- launchers of the engine kernels, shared by the host API (mb_api.cu) and the two
-// kernel translation units (mb_f64.cu: FP64 form, built without FMA contraction; mb_f32.cu: mixed
-// form, FP32 flux arithmetic with FMA).
+// mb_launch.h -- launchers of the engine kernels, shared by the host API (mb_api.cu) and the kernel translation units
+// (mb_f64.cu: per-cell and ghost kernels, built without FMA contraction; mb_sweep_*.cu: sweeps and records per form and
+// solver; mb_irs.cu, mb_prec.cu).
 #pragma once
 #include <cuda_runtime.h>
 #include "mb_engine.cuh"
@@ -36,7 +36,8 @@ struct GhostLists {
 };
 
 constexpr int TY_F64 = 5;    // tile rows of the FP64 parity sweep: 160 threads at 168 registers, 10 warps per SM; 4 rows
-                             // (232 registers, 8 warps) took 1.37 ms for a step of 64^3, these 1.07 ms; 160^3 the same
+                             // (232 registers, 8 warps) took 1.37 ms for a step of 64^3, these 1.07 ms; 160^3 the same.
+                             // The run-time solver unit, HLLE: 96^3 4.08 and 3.17 ms (its 5 rows spill up to 132 bytes)
 constexpr int TY_F64F = 8;   // tile rows of the FP64 production sweep: 256 threads at 128 registers, 16 warps per SM and an
                              // eighth of the j-faces computed twice. A step of 96^3: 4 rows (128 threads, 232 registers,
                              // 8 warps per SM) 1.71 ms, 6 rows (168 registers, 12 warps) 1.27 ms, 8 rows 1.14 ms

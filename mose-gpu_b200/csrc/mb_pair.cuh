@@ -56,13 +56,15 @@ __device__ __forceinline__ V2<float> fma2(V2<float> a, V2<float> b, V2<float> c)
   return r;
 }
 
-// reciprocal and square root of the flux path
+// reciprocal of the flux path. In FP32 within 1 ulp, 0 for |x| > 2^126 (the result would be subnormal) and infinite below
+// 2^-126. No denominator of the path comes near either end before the terms beside it overflow: densities are at least
+// 1e-20, the smallest sums carry 1e-30, and van Albada's squares reach 2^126 at slopes of 9e18, where its cubes have been
+// infinite since 7e12.
 __device__ __forceinline__ double rcp_(double x) { return 1.0 / x; }
 __device__ __forceinline__ float rcp_(float x) {
   float r;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
   return r;
 }
-
 
 }  // namespace mb

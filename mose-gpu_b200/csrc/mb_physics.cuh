@@ -162,7 +162,7 @@ struct Params {
                            // 2-D tensor of (ncell_total rows, 5 variables), or null (the same tile by plain loads)
   int* queue;              // persistent sweep: the tile counter (null: one CTA per tile)
   int ntiles_run;          // tiles of the launch (persistent sweep)
-  int chain;               // the launches of a stage are chained (launch_chained): the mesh has at most one tile per SM
+  int chain;               // the launches of a stage are chained (launch_chained): the smallest meshes (set_chain)
   int dense;               // 3-D mixed sweep at 4 CTAs per SM (64 registers) instead of 3 (80); its persistent grid
   int pgrid_dense;
   int pgrid;               // CTAs of a persistent launch (resident CTAs per SM x SMs)
