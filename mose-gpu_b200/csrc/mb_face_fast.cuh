@@ -186,10 +186,10 @@ __device__ __forceinline__ void roe_pair(const Params& p, const Side<R>& L, cons
 }
 
 // HLLC with the Batten signal speeds (hllc of mb_physics.cuh): the star state of the one side the contact selects. Its
-// flux F + S (U* - U) is written out: with r = 1 / (S - S*) the mass flux is rho (S - un) S* r, the velocity's weight is
-// that, and every other term is a small difference du = S* - un or the star pressure's, so no large terms cancel. The
-// rms error of the FP32 mass and energy fluxes over random states, against FP64: 7.4e-8 and 8.1e-8; summed as
-// F + S (U* - U) 2.5e-7 and 3.3e-7.
+// flux F + S (U* - U) is written out: with du = S* - un, m = rho (S - un) and the mass flux fr = m S* / (S - S*), the
+// pressure is p + g and the energy flux fr h0 + S* g, g = du (fr + m), so no large terms cancel (du = 0 gives F). The rms
+// error of the FP32 mass, momentum and energy fluxes over random subsonic states, against FP64: 7.4e-8, 3.7e-8 and 9.3e-8;
+// summed as F + S (U* - U) 2.6e-7, 4.5e-8 and 3.3e-7.
 template <typename R>
 __device__ __forceinline__ void hllc_pair(const Params& p, const Side<R>& L, const Side<R>& Q, R nx, R ny, R nz, R& fr,
                                           V2<R>& fuv, R& fw, R& fe) {
@@ -216,18 +216,17 @@ __device__ __forceinline__ void hllc_pair(const Params& p, const Side<R>& L, con
   // (S1 >= 0: the left flux; otherwise the side of the contact, with its physical flux alone where S4 <= 0)
   const bool left = S1 >= (R)0 || Ss >= (R)0;
   const R S = left ? S1 : S4;
-  const R un_ = left ? unL : unR, pk = left ? L.p : Q.p, w = left ? L.w : Q.w, e0 = left ? eL + kL : eR + kR;
+  const R un_ = left ? unL : unR, w = left ? L.w : Q.w, h0 = left ? h0L : h0R;
   const R mk = left ? mL : mR;  // rho (S - un)
   const V2<R> A = left ? L.A : Q.A;
   const bool star = left ? S1 < (R)0 : S4 > (R)0;
-  const R r = star ? rcp_(S - Ss) : (R)0;
-  const R du = star ? Ss - un_ : (R)0, vs = star ? Ss : un_;
-  const R ps = pk + mk * du;  // the star pressure, from the side's own state
-  fr = star ? mk * Ss * r : (left ? L.rho : Q.rho) * un_;
-  const R cn = ps + fr * du;
+  const R du = star ? Ss - un_ : (R)0;
+  fr = star ? mk * Ss * rcp_(S - Ss) : (left ? L.rho : Q.rho) * un_;
+  const R g = du * (fr + mk);
+  const R cn = (left ? L.p : Q.p) + g;
   fuv = fma2(dup2<R>(fr), A, dup2<R>(cn) * mk2<R>(nx, ny));
   fw = fr * w + cn * nz;
-  fe = fr * (e0 + du * Ss) + vs * (ps + pk * du * r);
+  fe = fr * h0 + Ss * g;
 }
 
 // AUSM+ (riemann_open of mb_physics.cuh, id 4)
