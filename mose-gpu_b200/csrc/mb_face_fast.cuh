@@ -98,6 +98,13 @@ __device__ __forceinline__ V2<double> albada(V2<double> a, V2<double> b, V2<doub
   right = V2<double>{b.x * c.x * (b.x + c.x) * (r01 * d0), b.y * c.y * (b.y + c.y) * (r23 * d2)};
   return V2<double>{b.x * a.x * (b.x + a.x) * (r01 * d1), b.y * a.y * (b.y + a.y) * (r23 * d3)};
 }
+// the same of one variable
+__device__ __forceinline__ double albada(double a, double b, double c, double& right) {
+  const double bb = b * b, d0 = fma(a, a, bb) + 1e-30, d1 = fma(c, c, bb) + 1e-30;
+  const double r = 1.0 / (d0 * d1);
+  right = b * c * (b + c) * (r * d0);
+  return b * a * (b + a) * (r * d1);
+}
 __device__ __forceinline__ V2<float> albada(V2<float> a, V2<float> b, V2<float> c, V2<float>& right) {
   const V2<float> bb = fma2(b, b, dup2<float>(1e-30f));
   const V2<float> dl = fma2(a, a, bb), dr = fma2(c, c, bb);
@@ -348,8 +355,24 @@ __device__ __forceinline__ void face_core(const Params& p, const DBlk& b, int d,
 #pragma unroll
     for (int q = 0; q < 4; ++q) c.stencil(q, A[q], B[q], C[q]);
     face_states(A[0], A[1], A[2], A[3], L.A, Q.A);
-    face_states(B[0], B[1], B[2], B[3], l, r);
-    L.w = lo2(l); Q.w = lo2(r);
+    if constexpr (sizeof(R) == 4) {  // w beside a T that nobody reads: the halves are independent
+      face_states(B[0], B[1], B[2], B[3], l, r);
+      L.w = lo2(l); Q.w = lo2(r);
+    } else {
+      // w alone: the pair's one division would mix in T, which has no value where a ghost that nothing fills is read (the
+      // second layer of a periodic axis one cell deep, a face without records: zero density), and w would have none either
+      const R a = (lo2(B[1]) - lo2(B[0])) * i0, e = (lo2(B[2]) - lo2(B[1])) * i1, f = (lo2(B[3]) - lo2(B[2])) * i2;
+      R sl, sr;
+      if (LIM == 3) {
+        sl = albada(a, e, f, sr);
+      } else {
+        const int lim = LIM ? LIM : p.lim;
+        sl = slope_rt<R>(lim, e, a);
+        sr = slope_rt<R>(lim, f, e);
+      }
+      L.w = fma(sl, (R)0.5 * dl1, lo2(B[1]));
+      Q.w = fma(sr, (R)-0.5 * dl2, lo2(B[2]));
+    }
     face_states(C[0], C[1], C[2], C[3], l, r);
     L.rho = mx(lo2(l), (R)1e-20); Q.rho = mx(lo2(r), (R)1e-20);
     L.p = hi2(l); Q.p = hi2(r);

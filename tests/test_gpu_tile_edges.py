@@ -220,3 +220,40 @@ def test_wall_friction_below_an_ulp_of_the_pressure_is_kept(engine):
     scale = np.abs(diff[0]).max()
     assert 0 < scale < 1e5 / 40 ** 2 * 6e-8  # below an ulp of the pressure force
     assert np.abs(diff[1] - diff[0]).max() < 1e-5 * scale, (np.abs(diff[1]).max(), scale)
+
+
+@pytest.mark.parametrize("riemann,limiter", [(abi.RS_LMROE, abi.LIM_VANALBADA), (abi.RS_HLLC, abi.LIM_VANALBADA),
+                                             (abi.RS_AUSMP, abi.LIM_VANALBADA), (abi.RS_HLLC, abi.LIM_MC)])
+@pytest.mark.parametrize("n,visc", [((24, 20, 1), 1), ((33, 9, 1), 0), ((20, 1, 24), 1), ((1, 24, 20), 1)])
+def test_periodic_axis_one_cell_deep(engine, n, visc, riemann, limiter):
+    """The second ghost layer of a periodic axis one cell deep comes from no interior cell and may hold zeros: the faces
+    beside it read no temperature from there."""
+    from mosegpu import case as cs
+    th = cs.ideal_gas_tables(mu=2e-2)
+    h = [1.0 / q for q in n]
+
+    def prim(c):
+        x, y, z = (2 * np.pi * c[..., q] * (n[q] > 1) for q in range(3))
+        return np.stack([1.0 + 0.1 * np.sin(x) * np.cos(y + z), 30 * np.sin(y) * np.cos(z), 20 * np.cos(x + z),
+                         10 * np.sin(x + y), 8.0e4 + 2e3 * np.cos(y + z)])
+    sch = dict(limiter=limiter, riemann=riemann, visc=visc, n_rk=3, ndir=3, cfl=0.3, prandtl=0.71, dt_additive=1)
+    case = cs.layout_case("slab", [[0, q] for q in n], lambda i, j, k: np.stack([i * h[0], j * h[1], k * h[2]], axis=-1),
+                          (True,) * 3, {}, th, sch, prim)
+    _steps(engine, case, abi.PREC_FP64, 1e-12)
+    _steps(engine, case, abi.PREC_FP64_FAST, 1e-12)
+    _steps(engine, case, abi.PREC_MIXED, 3e-6)
+
+
+@pytest.mark.parametrize("riemann", [abi.RS_LMROE, abi.RS_HLLC, abi.RS_AUSMP])
+def test_a_face_without_records_beside_empty_ghosts(engine, riemann):
+    """No record, no flux and no ghosts: the faces next to such a boundary reach cells of zero density, whose temperature is
+    not a number, and keep finite fluxes as in the parity form."""
+    from mosegpu import case as cs
+    case = cs.multiblock_2d(cols=1, rows=1, widths=[35], heights=[9], visc=0, mach=0.5, n_rk=3, cfl=0.2, riemann=riemann,
+                            limiter=abi.LIM_VANALBADA, bc={1: abi.BC_INFLOW, 2: abi.BC_EXTRAPOLATION, 3: abi.BC_WALL,
+                                                           4: abi.BC_EXTRAPOLATION, 5: abi.BC_EXTRAPOLATION,
+                                                           6: abi.BC_EXTRAPOLATION})
+    case.rec = case.rec[case.rec["face"] != 4].copy()
+    case.P0 = np.where(case.interior_mask()[None], case.P0, 0.0)
+    _steps(engine, case, abi.PREC_FP64, 1e-12, exact=True)
+    _steps(engine, case, abi.PREC_FP64_FAST, 1e-12)
