@@ -1149,7 +1149,7 @@ MB_HD void hlle_flux(R ul, R vl, R wl, R pl, R dltot, R h0l, R ur, R vr, R wr, R
 }
 
 // SLAU at the boundary records (Lib_Riemann.f90:140-197): T = p / (rho R) and H0 = h(T) + V^2/2 of each state from
-// the tables (no T clamp), then the SLAU flux
+// the tables (no clamp there; the row is held to the table here), then the SLAU flux
 template <typename R>
 MB_HD void slau_rec(const Params& p, R dl, R ul, R vl, R wl, R pl, R al, R dltot, R dr, R ur, R vr, R wr, R pr, R ar,
                     R drtot, R nx, R ny, R nz, R& F_r, R& F_u, R& F_v, R& F_w, R& F_E) {
@@ -1160,7 +1160,7 @@ MB_HD void slau_rec(const Params& p, R dl, R ul, R vl, R wl, R pl, R al, R dltot
   R Rl = (R)0 + ri * dl / dltot;
   R Rr = (R)0 + ri * dr / drtot;
   R Tl = pl / (dltot * Rl), Tr = pr / (drtot * Rr);
-  int Til = (int)Tl, Tir = (int)Tr;
+  int Til = tidx(p, Tl), Tir = tidx(p, Tr);
   R dTl = Tl - (R)Til, dTr = Tr - (R)Tir;
   R h0l = (R)0 + (H[Til] + (H[Til + 1] - H[Til]) * dTl) * dl / dltot;
   R h0r = (R)0 + (H[Tir] + (H[Tir + 1] - H[Tir]) * dTr) * dr / drtot;

@@ -969,7 +969,7 @@ void riemann_hllc_bc(const Thermo& th, int rs, double dl, double ul, double vl, 
 }
 
 // SLAU at the records (Lib_Riemann.f90:140-197): T = p / (rho R) and H0 = h(T) + V^2/2 of each state from the
-// tables (no T clamp), then the SLAU flux
+// tables (no clamp there; the row is held to the table here), then the SLAU flux
 void riemann_slau_bc(const Thermo& th, double dl, double ul, double vl, double wl, double pl, double al, double dltot,
                      double dr, double ur, double vr, double wr, double pr, double ar, double drtot, double nx,
                      double ny, double nz, double& F_r, double& F_u, double& F_v, double& F_w, double& F_E) {
@@ -978,7 +978,7 @@ void riemann_slau_bc(const Thermo& th, double dl, double ul, double vl, double w
   double Rl = 0.0 + th.ri * dl / dltot;
   double Rr = 0.0 + th.ri * dr / drtot;
   double Tl = pl / (dltot * Rl), Tr = pr / (drtot * Rr);
-  int Til = (int)Tl, Tir = (int)Tr;
+  int Til = tidx(th, Tl), Tir = tidx(th, Tr);
   double dTl = Tl - Til, dTr = Tr - Tir;
   double h0l = 0.0 + (th.h[Til] + (th.h[Til + 1] - th.h[Til]) * dTl) * dl / dltot;
   double h0r = 0.0 + (th.h[Tir] + (th.h[Tir + 1] - th.h[Tir]) * dTr) * dr / drtot;
