@@ -194,9 +194,10 @@ __device__ __forceinline__ void roe_pair(const Params& p, const Side<R>& L, cons
 
 // HLLC with the Batten signal speeds (hllc of mb_physics.cuh): the star state of the one side the contact selects. Its
 // flux F + S (U* - U) is written out: with du = S* - un, m = rho (S - un) and the mass flux fr = m S* / (S - S*), the
-// pressure is p + g and the energy flux fr h0 + S* g, g = du (fr + m), so no large terms cancel (du = 0 gives F). The rms
-// error of the FP32 mass, momentum and energy fluxes over random subsonic states, against FP64: 7.4e-8, 3.7e-8 and 9.3e-8;
-// summed as F + S (U* - U) 2.6e-7, 4.5e-8 and 3.3e-7.
+// pressure is p + g and the energy flux fr h0 + S* g, g = du (fr + m), so no large terms cancel. du = S* = 0 gives F, which
+// takes nothing from the other side: a supersonic face stays finite beside a state that is not. The rms error of the FP32
+// mass, momentum and energy fluxes over random subsonic states, against FP64: 7.4e-8, 3.7e-8 and 9.3e-8; summed as
+// F + S (U* - U) 2.6e-7, 4.5e-8 and 3.3e-7.
 template <typename R>
 __device__ __forceinline__ void hllc_pair(const Params& p, const Side<R>& L, const Side<R>& Q, R nx, R ny, R nz, R& fr,
                                           V2<R>& fuv, R& fw, R& fe) {
@@ -227,13 +228,13 @@ __device__ __forceinline__ void hllc_pair(const Params& p, const Side<R>& L, con
   const R mk = left ? mL : mR;  // rho (S - un)
   const V2<R> A = left ? L.A : Q.A;
   const bool star = left ? S1 < (R)0 : S4 > (R)0;
-  const R du = star ? Ss - un_ : (R)0;
+  const R du = star ? Ss - un_ : (R)0, Sx = star ? Ss : (R)0;
   fr = star ? mk * Ss * rcp_(S - Ss) : (left ? L.rho : Q.rho) * un_;
   const R g = du * (fr + mk);
   const R cn = (left ? L.p : Q.p) + g;
   fuv = fma2(dup2<R>(fr), A, dup2<R>(cn) * mk2<R>(nx, ny));
   fw = fr * w + cn * nz;
-  fe = fr * h0 + Ss * g;
+  fe = fr * h0 + Sx * g;
 }
 
 // AUSM+ (riemann_open of mb_physics.cuh, id 4)

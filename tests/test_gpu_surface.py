@@ -123,3 +123,21 @@ def test_a_value_that_is_not_finite_stays_within_its_stencil(engine, at, bad, pr
     far = ~(((di <= 2) & (dj == 0)) | ((dj <= 2) & (di == 0)))
     assert np.array_equal(res[0][:, far], res[1][:, far])
     assert not np.isfinite(res[1][:, at[0], at[1]]).all()
+
+
+@pytest.mark.parametrize("precision", [abi.PREC_FP64, abi.PREC_FP64_FAST, abi.PREC_MIXED])
+def test_a_supersonic_hllc_face_takes_nothing_from_downstream(engine, precision):
+    """At Mach 2 the flux of a face is its left state's. A cell that is not a number spoils the right state of the face two
+    cells upstream and the states of the next one: the residual two cells upstream keeps its bits."""
+    case = _channel(70, 20, (E, E, E, E), 0, mach=2.0)
+    P = case.P0.copy()
+    case.interior(P, 0)[4, 33, 9, 0] = np.nan
+    res = []
+    for state in (case.P0, P):
+        eng = engine(case, precision=precision)
+        eng.set_state(state)
+        eng.fill_ghosts()
+        res.append(case.interior(eng.residual().cpu().numpy(), 0)[:, :, 9, 0])
+        eng.close()
+    assert np.array_equal(res[0][:, :32], res[1][:, :32])
+    assert not np.isfinite(res[1][:, 32]).all()
