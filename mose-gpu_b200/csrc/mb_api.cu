@@ -573,6 +573,19 @@ static int build_tables(mb_ctx* c, const mb_mesh* mesh) {
     kca /= 2;
     ta = make_tiles(c->hdims, TY_AUX, kca, 0xe, &c->hkm, -1);
   }
+  // a donor one cell deep hands its first ghost layer on as its second: the first layers of all go first
+  int ncopy1 = 0;
+  if (!deep_donors) {
+    std::vector<long long> d2, s2;
+    for (int l = 0; l < MB_GC; ++l)
+      for (size_t q = l; q < cdst.size(); q += MB_GC) {
+        d2.push_back(cdst[q]);
+        s2.push_back(csrc[q]);
+      }
+    cdst.swap(d2);
+    csrc.swap(s2);
+    ncopy1 = (int)cdst.size() / MB_GC;
+  }
   // ---- the mixed form reads its geometry in FP32: one conversion per distinct array of this mesh (blocks may
   // share arrays). Every copy is converted afresh (a caller may have replaced an array at the same address);
   // the buffers of the previous mesh are reused where the size matches.
@@ -702,7 +715,7 @@ static int build_tables(mb_ctx* c, const mb_mesh* mesh) {
   p.recflux = c->d_recflux;
   GhostLists& g = c->g;
   g.rec = c->d_grec; g.phys = c->d_phys; g.nphys = (int)phys.size(); g.cubic = c->d_cubic; g.ncubic = (int)cubic.size();
-  g.cdst = c->d_cdst; g.csrc = c->d_csrc; g.ncopy = (int)cdst.size(); g.pgsrc = c->d_pgsrc; g.nconn = mesh->nconn;
+  g.cdst = c->d_cdst; g.csrc = c->d_csrc; g.ncopy = (int)cdst.size(); g.ncopy1 = ncopy1; g.pgsrc = c->d_pgsrc; g.nconn = mesh->nconn;
   g.ordered = ordered;
   g.fused = !ordered && deep_donors && !lone;
   bool reads_ghosts = false;  // a record of the work list reads a ghost row

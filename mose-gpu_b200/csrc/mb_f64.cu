@@ -98,7 +98,8 @@ __global__ void k_ghost_cubic(Params p, const GRec* __restrict__ rec, const int*
 }
 
 // 1:1 and periodic connections (Ghost_Connection_pair, :1023-1134): receiver ghost layer g <- donor layer g.
-// The donor layers are interior cells, so the copies of one launch never read what another writes.
+// The donor layers are interior cells, so the copies of one launch never read what another writes; the second layer of a
+// donor one cell deep is its own first ghost layer, so there the first layers are copied by a launch of their own.
 __global__ void k_ghost_copy(const long long* __restrict__ dst, const long long* __restrict__ src, int n, long long nc,
                              double* P) {
   long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -213,8 +214,8 @@ cudaError_t ghost_fill(const Params& p, const GhostLists& g, double* P, cudaStre
       if (n > 0) { k_ghost_cubic<<<nblk_for(n, 128), 128, 0, s>>>(p, g.rec, g.cubic + g.cubic_off[f], n, P); ++*nl; }
     }
   }
-  if (g.ncopy > 0) {
-    k_ghost_copy<<<nblk_for((long long)g.ncopy * MB_NP, 256), 256, 0, s>>>(g.cdst, g.csrc, g.ncopy, p.nc, P);
+  for (int lo = 0, n = g.ncopy1 > 0 ? g.ncopy1 : g.ncopy; n > 0; lo += n, n = g.ncopy - lo) {
+    k_ghost_copy<<<nblk_for((long long)n * MB_NP, 256), 256, 0, s>>>(g.cdst + lo, g.csrc + lo, n, p.nc, P);
     ++*nl;
   }
   return cudaGetLastError();

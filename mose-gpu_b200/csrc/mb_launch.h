@@ -17,6 +17,7 @@ struct GhostLists {
   const long long* cdst;  // connection ghost copies: row cdst[q] <- row csrc[q]
   const long long* csrc;
   int ncopy;
+  int ncopy1;             // where a donor is one cell deep: the first-layer copies, ahead of the others and launched alone
   const long long* pgsrc; // [nconn][6] source rows of bc_pg
   int nconn;
   // ordered != 0: the phys and cubic lists are split in two halves, off[0]..off[1] and off[1]..off[2], the second
